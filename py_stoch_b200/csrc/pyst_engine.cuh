@@ -306,6 +306,24 @@ __device__ __forceinline__ int pnet_delta(uint32_t d, int q) {
 }
 __device__ __forceinline__ int pnet_count(uint32_t d) { return (int)(d >> 30); }
 
+// acc + (double)a for a >= 0 (the sign of a zero is dropped: it does not
+// change the sum).  The float's bits shifted into a double's fields are
+// a 2^-896, subnormals and zero included, and the fused multiply-add scales
+// them back exactly, so no conversion instruction (23 cycles of latency, an
+// eighth of the issue rate) is on a step's dependent chain.  An infinite or
+// NaN a adds 2^128 or more: callers test sums against PYST_RATE_BIG.
+#define PYST_RATE_BIG 0x1.0p128
+__device__ __forceinline__ double add_rate(double acc, float a) {
+  const uint32_t u = __float_as_uint(a) & 0x7FFFFFFFu;
+  return __fma_rn(__hiloint2double((int)(u >> 3), (int)(u << 29)),
+                  0x1.0p896, acc);
+}
+// Whether a sum of add_rate terms is neither zero nor at PYST_RATE_BIG
+// (for a sum >= 0, by its high word).
+__device__ __forceinline__ bool rate_sum_usable(double a0) {
+  return (uint32_t)__double2hiint(a0) - 1u < 0x47F00000u - 1u;
+}
+
 __device__ __forceinline__ void store_sample(const TrajOut& o, int ita, int k,
                                              int f, int32_t v) {
   o.samples[((int64_t)k * ita + f) * o.stride] = v;
@@ -428,11 +446,28 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
   }
   double t = st.t;
   int f = st.f;
+  // steps and events of this call in 32 bits (nst; the events of its
+  // direct-method steps are their number), folded into the 64-bit counts at
+  // its end or when nst reaches `lim`, the step budget or 2^30
   int64_t events = st.events, steps = st.steps;
+  int nst = 0, n_ssa = 0, n_leap = 0;
+  auto steps_left = [&]() {
+    const int64_t left = ra.step_budget - steps;
+    return (int)(left < (1ll << 30) ? left : (1ll << 30));
+  };
+  int lim = steps_left();
+  // out of steps?  (folds the counts when only the 32-bit range is used up)
+  auto budget_spent = [&]() {
+    steps += nst;
+    events += n_ssa;
+    nst = n_ssa = 0;
+    lim = steps_left();
+    return lim <= 0;
+  };
   uint64_t h = st.h;
+  const bool want_h = o.seqhash != nullptr;
   int status = PYST_TRAJ_DONE;
   bool fill_state = false, done = false;
-  const int64_t budget = ra.step_budget;
   const double t_end = m.time(ita - 1);
   double tf = m.time(f);  // next sample time (f < ita while running)
   static_assert(GROUP == kGroupAny || TAU, "groups: tau-leaping only");
@@ -444,7 +479,6 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
   bool leap_grp = group_leap;
   int ssa_left = st.ssa_left;
   uint32_t leap_q = st.leap_q;
-  int n_ssa = 0, n_leap = 0;
   auto xget = [&](int i) { return XV(i); };
 
   while (true) {
@@ -452,17 +486,20 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
     // DECIDE before stopping, so the slot's next round is in the group of
     // its outcome (it would otherwise spend that round only switching).
     // (Leap-group rounds do not: their slots would run every continuing
-    // leap's DECIDE twice.)
-    const bool capped = n_ssa >= cap_ssa || n_leap >= cap_leap;
+    // leap's DECIDE twice.)  Whole-trajectory calls have no caps.
+    const bool capped = GROUP == kGroupSsa ? n_ssa >= cap_ssa
+                        : GROUP == kGroupLeap ? n_leap >= cap_leap : false;
     if (capped && !(GROUP == kGroupSsa && !ssa_mode)) break;
     float a[MAXR];
+    double P[MAXR];  // prefix sums of the propensities, P[R - 1] the total
     double a0 = 0.0;
 #pragma unroll
     for (int j = 0; j < MAXR; ++j) {
       if (j >= R) break;
       a[j] = pk ? propensity_packed(m.rate(j), m.pk[j], xget)
                     : propensity<kLaws>(m, j, xcol, bs);
-      a0 = __dadd_rn(a0, (double)a[j]);
+      a0 = add_rate(a0, a[j]);
+      P[j] = a0;
     }
     if (kLaws && m.nlaw) {
       bool bad = false;
@@ -477,19 +514,27 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
         break;
       }
     }
-    if (a0 == 0.0) {
-      status = PYST_TRAJ_ABSORBED;
-      fill_state = true;
-      done = true;
-      break;
-    }
-    if (steps >= budget) {
-      status = PYST_TRAJ_STEP_BUDGET;
-      done = true;
-      break;
-    }
     if (TAU && (GROUP == kGroupLeap || !ssa_mode)) {
       // ---------------- DECIDE: critical set, tau_1, SSA switch -------
+      if (!rate_sum_usable(a0)) {
+        if (a0 == 0.0) {
+          status = PYST_TRAJ_ABSORBED;
+          fill_state = true;
+          done = true;
+          break;
+        }
+        a0 = 0.0;  // an infinite or NaN propensity: plain conversions
+#pragma unroll
+        for (int j = 0; j < MAXR; ++j) {
+          if (j >= R) break;
+          a0 = __dadd_rn(a0, (double)a[j]);
+        }
+      }
+      if (nst >= lim && budget_spent()) {
+        status = PYST_TRAJ_STEP_BUDGET;
+        done = true;
+        break;
+      }
       uint32_t crit = 0u;
 #pragma unroll
       for (int j = 0; j < MAXR; ++j) {
@@ -559,7 +604,7 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
         if (capped || GROUP == kGroupSsa || (stop_on_switch && !group_leap))
           break;
         // ---------------- leap ---------------------------------------
-        steps++;
+        nst++;
         n_leap++;
         double a0c = 0.0;
 #pragma unroll
@@ -684,12 +729,13 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
         leap_q++;
         const double tn = __dadd_rn(t, tau);
         int64_t fired = 0;
-        h = seq_mix(h, PYST_LEAP_TAG);
+        if (want_h) h = seq_mix(h, PYST_LEAP_TAG);
 #pragma unroll
         for (int j = 0; j < MAXR; ++j) {
           if (j >= R) break;
           fired += K[j];
-          if (K[j] != 0) h = seq_mix(h, ((uint64_t)j << 32) | (uint32_t)K[j]);
+          if (want_h && K[j] != 0)
+            h = seq_mix(h, ((uint64_t)j << 32) | (uint32_t)K[j]);
           if (SCORE) {
             cnt[j] += K[j];
             integ[j] = __dadd_rn(integ[j], __dmul_rn((double)a[j], tau));
@@ -717,14 +763,14 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
       }
     }
     // ------------------------ one direct-method step -------------------
-    steps++;
-    n_ssa++;
-    double tau, r;
+    // The propensities above, the clock, the next step's random numbers and
+    // the selection are one straight line of code, so that their chains
+    // overlap; everything rare (a zero or infinite total, the step budget,
+    // a sample time passed) is behind the one test at its end.
+    double e, uu;
     if constexpr (LG > 1) {
-      const double e = __shfl_sync(g_mask, g_e, g_i, LG);
-      const double uu = __shfl_sync(g_mask, g_u, g_i, LG);
-      tau = __ddiv_rn(e, a0);
-      r = __dmul_rn(uu, a0);
+      e = __shfl_sync(g_mask, g_e, g_i, LG);
+      uu = __shfl_sync(g_mask, g_u, g_i, LG);
       if (++g_i == LG) {
         g_i = 0;
         g_base += LG;
@@ -734,31 +780,71 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
         g_u = u53(wg.z, wg.w);
       }
     } else {
-      const uint4 w = w_pf;
-      tau = __ddiv_rn(e_pf, a0);
+      e = e_pf;
+      uu = u53(w_pf.z, w_pf.w);
       w_pf = next_block(rs);
       e_pf = -pyst_log(u53(w_pf.x, w_pf.y));
-      r = __dmul_rn(u53(w.z, w.w), a0);
     }
-    int sel = -1;
-    {
-      double cum = 0.0;
-      int lastnz = -1;
+    double tau = ddiv_normal(e, a0);
+    // the first j whose prefix sum reaches r: r <= a0 = P[R - 1] (uu <= 1)
+    // and the sums do not decrease, so it is the number of sums below r,
+    // and a[sel] > 0
+    const double r = __dmul_rn(uu, a0);
+    int sel = 0;
 #pragma unroll
-      for (int j = 0; j < MAXR; ++j) {
-        if (j >= R) break;
-        cum = __dadd_rn(cum, (double)a[j]);
-        if (a[j] > 0.0f) lastnz = j;
-        if (cum >= r) {
-          sel = j;
+    for (int j = 0; j < MAXR - 1; ++j) {
+      if (j >= R - 1) break;
+      sel += P[j] < r ? 1 : 0;
+    }
+    double tn = __dadd_rn(t, tau);
+    if (!rate_sum_usable(a0) || tn >= tf || nst >= lim) {
+      if (a0 == 0.0) {
+        status = PYST_TRAJ_ABSORBED;
+        fill_state = true;
+        done = true;
+        break;
+      }
+      if (nst >= lim && budget_spent()) {
+        status = PYST_TRAJ_STEP_BUDGET;
+        done = true;
+        break;
+      }
+      if (!rate_sum_usable(a0)) {
+        // an infinite or NaN propensity: plain conversions and division
+        a0 = 0.0;
+#pragma unroll
+        for (int j = 0; j < MAXR; ++j) {
+          if (j >= R) break;
+          a0 = __dadd_rn(a0, (double)a[j]);
+        }
+        tau = __ddiv_rn(e, a0);
+        tn = __dadd_rn(t, tau);
+        const double rx = __dmul_rn(uu, a0);
+        double cum = 0.0;
+        int lastnz = -1;
+        sel = -1;
+#pragma unroll
+        for (int j = 0; j < MAXR; ++j) {
+          if (j >= R) break;
+          cum = __dadd_rn(cum, (double)a[j]);
+          if (a[j] > 0.0f) lastnz = j;
+          if (sel < 0 && cum >= rx) sel = j;
+        }
+        if (sel < 0) sel = lastnz;
+      }
+      while (tn >= tf) {
+        if (LG == 1 || g_lane == 0)
+          for (int k = 0; k < kappa; ++k)
+            store_sample(o, ita, k, f, XV(m.out(k)));
+        f++;
+        if (f == ita) {
+          done = true;
           break;
         }
+        tf = m.time(f);
       }
-      // unreachable in exact arithmetic (the last sum equals a0 >= r);
-      // kept so a selection always names a reaction with a_j > 0
-      if (sel < 0) sel = lastnz;
     }
-    const double tn = __dadd_rn(t, tau);
+    nst++;
     if (SCORE) {
       const double dt = (tn >= t_end) ? __dsub_rn(t_end, t) : tau;
 #pragma unroll
@@ -767,20 +853,10 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
         integ[j] = __dadd_rn(integ[j], __dmul_rn((double)a[j], dt));
       }
     }
-    while (tn >= tf) {
-      if (LG == 1 || g_lane == 0)
-        for (int k = 0; k < kappa; ++k)
-          store_sample(o, ita, k, f, XV(m.out(k)));
-      f++;
-      if (f == ita) {
-        done = true;
-        break;
-      }
-      tf = m.time(f);
-    }
     t = tn;
     if (done) break;
     {
+      // counts stay in [0, 2^31): a step outside wraps to a negative number
       bool over = false;
       if (pk) {
         const uint32_t d = m.pk[R + sel];
@@ -788,9 +864,10 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
         for (int q = 0; q < 2; ++q) {
           if (q < pnet_count(d)) {
             const int sp = pnet_species(d, q);
-            const int64_t nx = (int64_t)XV(sp) + pnet_delta(d, q);
-            if (nx < 0 || nx > PYST_I32MAX) over = true;
-            else XV(sp) = (int)nx;
+            const int nx =
+                (int)((uint32_t)XV(sp) + (uint32_t)pnet_delta(d, q));
+            if (nx < 0) over = true;
+            else XV(sp) = nx;
           }
         }
       } else {
@@ -798,9 +875,9 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
         for (int e = m.netptr(sel); e < e1; ++e) {
           const uint32_t ne = m.net(e);
           const int sp = ent_lo(ne);
-          const int64_t nx = (int64_t)XV(sp) + ent_hi_s16(ne);
-          if (nx < 0 || nx > PYST_I32MAX) over = true;
-          else XV(sp) = (int)nx;
+          const int nx = (int)((uint32_t)XV(sp) + (uint32_t)ent_hi_s16(ne));
+          if (nx < 0) over = true;
+          else XV(sp) = nx;
         }
       }
       if (over) {
@@ -809,8 +886,8 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
         break;
       }
     }
-    events++;
-    h = seq_mix(h, (uint64_t)sel);
+    n_ssa++;  // (completed steps: each is one event)
+    if (want_h) h = seq_mix(h, (uint64_t)sel);
     if (SCORE) {
 #pragma unroll
       for (int j = 0; j < MAXR; ++j) cnt[j] += (j == sel) ? 1 : 0;
@@ -819,6 +896,8 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
       if (--ssa_left <= 0) ssa_mode = false;
     }
   }
+  events += n_ssa;
+  steps += nst;
   st.t = t;
   // the prefetched block (LG = 1) was not used
   st.n = LG > 1 ? g_base + (uint64_t)g_i : rs.n - 1;
