@@ -67,8 +67,12 @@ enum { PYST_MAP_AUTO = 0, PYST_MAP_THREAD = 1, PYST_MAP_WARP = 2 };
 
 /* pyst_run_desc.flags bits.  PYST_FLAG_UNSORTED: run thread-mapped
  * tau-leaping with the simple one-trajectory-per-thread loop instead of the
- * default mode-sorted block scheduler (same results, slower). */
-enum { PYST_FLAG_UNSORTED = 1 };
+ * default mode-sorted block scheduler (same results, slower).
+ * PYST_FLAG_LANE_GROUPS: batched runs of few trajectories: thread-mapped
+ * items of at most 8 small mass-action reactions run a group of lanes per
+ * trajectory instead of a thread (same results, faster while the batch does
+ * not fill the GPU). */
+enum { PYST_FLAG_UNSORTED = 1, PYST_FLAG_LANE_GROUPS = 2 };
 
 /* Limits of this library. */
 #define PYST_MAX_SPECIES 1024
@@ -237,7 +241,11 @@ typedef struct pyst_batch_limits {
   int32_t max_blob_words;
   int32_t max_species;
   int32_t max_reactions;
-  int32_t reserved;
+  int32_t reserved;  /* 0; with PYST_FLAG_LANE_GROUPS may be parts << 16 |
+                        part: blocks then share each item in `parts` parts of
+                        `part` trajectories (parts * part at least the
+                        largest item's), and `group` must be set, one per
+                        model, for unsplit models too                       */
 } pyst_batch_limits;
 
 /* Workspace bytes pyst_batch_run needs for n_items items: the work-queue

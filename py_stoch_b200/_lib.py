@@ -35,6 +35,7 @@ MAP_AUTO = 0
 MAP_THREAD = 1
 MAP_WARP = 2
 FLAG_UNSORTED = 1
+FLAG_LANE_GROUPS = 2
 
 MAX_SPECIES = 1024
 MAX_REACTIONS = 4096

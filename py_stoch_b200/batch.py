@@ -52,6 +52,13 @@ def auto_mapping(model, score=False):
     return _lib.MAP_THREAD
 
 
+def small_model(model):
+    """Models of the size the lane groups take (the kernel checks the
+    reactions themselves)."""
+    return (model.n_reactions <= 8 and model.n_species <= 8 and
+            not getattr(model, 'has_laws', False))
+
+
 class Batch(object):
     """A set of (model, trajectories, method, mapping) items."""
 
@@ -105,6 +112,7 @@ class Batch(object):
                                         _lib.THREAD_MAX_REACTIONS) else x
                       for m, x in zip(self.models, mp)]
         self.mappings = np.array(mp, np.int32)
+        self.lane_groups = bool(chunk) and self._use_lane_groups(torch)
         if traj_id_base is None:
             traj_id_base = np.concatenate([[0], np.cumsum(self.n_traj)[:-1]])
         self.traj_id_base = np.asarray(traj_id_base, np.int64)
@@ -181,6 +189,12 @@ class Batch(object):
             max(len(b) for b in blobs),
             max(m.n_species for m in self.models),
             max(m.n_reactions for m in self.models), 0)
+        if self.lane_groups:
+            # blocks share an item in parts of one trajectory per group
+            part = 32 if all(m.n_reactions <= 4 and m.n_species <= 4
+                             for m in self.models) else 16
+            parts = -(-int(self.item_n_traj.max(initial=1)) // part)
+            self.limits.reserved = min(parts, 0x7FFF) << 16 | part
         L = _lib.lib()
         ws = C.c_size_t(0)
         _lib.check(L.pyst_batch_workspace_size(self.n_items, C.byref(ws)),
@@ -214,6 +228,22 @@ class Batch(object):
                 int((2 * self.kappa * self.ita * self.R).sum()),
                 dtype=torch.float64, device=dev)
 
+    def _use_lane_groups(self, torch):
+        """Whether thread-mapped items run a lane group per trajectory: the
+        batch is far from filling the GPU thread by thread and at least half
+        of its trajectories are of models the lane groups take.  The lines
+        (trajectories per SM) are where the two forms meet: tau-leaping at
+        about 200, the direct method at about 96."""
+        ok = np.array([x == _lib.MAP_THREAD and small_model(m)
+                       for m, x in zip(self.models, self.mappings)], bool)
+        total = int(self.n_traj.sum())
+        if 2 * int(self.n_traj[ok].sum()) < max(total, 1):
+            return False
+        tau = bool((self.methods == _lib.METHOD_TAU_LEAP).all())
+        sms = torch.cuda.get_device_properties(
+            self.device).multi_processor_count
+        return total <= (200 if tau else 96) * sms
+
     def run(self, seed=0, stream=None, ssa_fallback_steps=100,
             max_leap_retries=63, step_budget=None, block_size=0):
         """Enqueue the whole batch on ``stream`` (one kernel launch).
@@ -222,7 +252,7 @@ class Batch(object):
         torch = _torch()
         L = _lib.lib()
         if not block_size:
-            block_size = 64 if int(self.item_n_traj.max()) <= 64 else 128
+            block_size = 128 if self.lane_groups else 64 if int(self.item_n_traj.max()) <= 64 else 128
         if step_budget is None:
             step_budget = DEFAULT_STEP_BUDGET
         o = self.out
@@ -237,7 +267,8 @@ class Batch(object):
             o['jacobian'].data_ptr() if 'jacobian' in o else 0)
         r = _lib.RunDesc(0, 0, int(seed) & 0xFFFFFFFFFFFFFFFF, 0, 0,
                          int(ssa_fallback_steps), int(max_leap_retries),
-                         int(step_budget), int(block_size), 0)
+                         int(step_budget), int(block_size),
+                         _lib.FLAG_LANE_GROUPS if self.lane_groups else 0)
         if stream is None:
             stream = torch.cuda.current_stream(self.device)
         _lib.check(L.pyst_batch_run(

@@ -5,8 +5,9 @@
 The library links these objects with the static CUDA runtime, so it loads
 on machines without a GPU (only the run calls need one):
 
-* pyst_k_thread.cu, pyst_k_warp.cu  x (PYST_TAU, PYST_SCORE) in {0,1}^2
-* pyst_k_batch.cu, pyst_k_sorted.cu x PYST_SCORE in {0,1}
+* pyst_k_thread.cu, pyst_k_warp.cu, pyst_k_group.cu x (PYST_TAU, PYST_SCORE) in {0,1}^2
+* pyst_k_batch.cu x (PYST_GROUPS, PYST_SCORE) in {0,1}^2
+* pyst_k_sorted.cu x (PYST_SCORE, PYST_PART) in {0,1} x {0..4}
 * pyst_k_misc.cu (gradient reduction, test hooks), pyst_capi.cu (C ABI)
 * pyst_pack.cpp (host-only model packer)
 
@@ -32,7 +33,7 @@ NVCC_FLAGS = ARCH + ['-O3', '-lineinfo', '--fmad=false', '-std=c++17',
                      '-Xcompiler', '-fPIC,-O2', '--expt-relaxed-constexpr']
 HEADERS = [os.path.join(CSRC, f) for f in
            ('pyst_engine.cuh', 'pyst_math.cuh', 'pyst_model.cuh',
-            'pyst_launch.cuh')] + [
+            'pyst_launch.cuh', 'pyst_group.cuh')] + [
     os.path.join(INCLUDE, 'pystoch_b200.h'),
     os.path.join(INCLUDE, 'pystoch_b200_testing.h')]
 
@@ -41,14 +42,16 @@ def units():
     out = []
     for t in (0, 1):
         for s in (0, 1):
-            for base in ('pyst_k_thread', 'pyst_k_warp'):
+            for base in ('pyst_k_thread', 'pyst_k_warp', 'pyst_k_group'):
                 out.append((base + '.cu', '%s_t%ds%d.o' % (base, t, s),
                             ['-DPYST_TAU=%d' % t, '-DPYST_SCORE=%d' % s]))
     for s in (0, 1):
-        out.append(('pyst_k_batch.cu', 'pyst_k_batch_s%d.o' % s,
-                    ['-DPYST_SCORE=%d' % s]))
-        out.append(('pyst_k_sorted.cu', 'pyst_k_sorted_s%d.o' % s,
-                    ['-DPYST_SCORE=%d' % s]))
+        for g in (0, 1):
+            out.append(('pyst_k_batch.cu', 'pyst_k_batch_g%ds%d.o' % (g, s),
+                        ['-DPYST_GROUPS=%d' % g, '-DPYST_SCORE=%d' % s]))
+        for part in range(5):
+            out.append(('pyst_k_sorted.cu', 'pyst_k_sorted_s%dp%d.o' % (
+                s, part), ['-DPYST_SCORE=%d' % s, '-DPYST_PART=%d' % part]))
     out.append(('pyst_k_misc.cu', 'pyst_k_misc.o', []))
     out.append(('pyst_capi.cu', 'pyst_capi.o', []))
     out.append(('pyst_pack.cpp', 'pyst_pack.o', []))

@@ -85,6 +85,7 @@ int read_header(const uint32_t* h, HostModelInfo* mi) {
   mi->packable = mi->nlaw == 0 && sections_in_blob(h, mi->words, mi->R);
   for (int j = 0; j < mi->R && mi->packable; ++j)
     mi->packable = blob_reaction_packable(h, j);
+  mi->factors = mi->packable ? blob_direct_factors(h) : 0;
   return PYST_OK;
 }
 
@@ -140,6 +141,33 @@ OutBase make_outbase(const pyst_outputs* out, int64_t n_traj) {
   return ob;
 }
 
+// Lanes per trajectory for a run of n trajectories (pyst_group.cuh), or 0 for
+// a thread per trajectory.  More lanes shorten a step while warps are few;
+// past that they cost issue slots.  The lines, in trajectories per SM, lie
+// where the next form measured faster (148 SMs, ms; t: thread form, for
+// tau-leaping the mode-sorted scheduler):
+//   direct, Lotka-Volterra: 1,184 32: 53 16: 48; 2,368 16: 55 8: 52;
+//     4,999 8: 70 4: 68 t: 119; 9,472 4: 70 t: 121; 20,011 4: 147 t: 142;
+//   direct, telegraph (6 reactions): 592 32: 2.0 16: 2.2; 2,368 16: 2.4
+//     8: 2.4; 9,472 8: 3.7 t: 5.0; 20,011 8: 7.1 t: 5.8;
+//   tau, Schlogl: 2,368 32: 5.1 16: 6.9; 4,999 32: 10.8 8: 9.4 4: 9.5;
+//     20,011 4: 15.6 t: 20.3; 40,000 4: 31.9 t: 20.3;
+//   tau, Lotka-Volterra: 2,368 32: 21.0 8: 20.9; 9,472 8: 27 4: 25;
+//     20,011 4: 33 t: 90; 40,000 4: 54 t: 93.
+int group_lanes(const HostModelInfo& mi, int64_t n, bool tau) {
+  if (mi.factors < 1 || mi.S > 32) return 0;
+  int least = mi.R > 4 || mi.S > 4 ? 8 : 4;
+  while (least < mi.S) least *= 2;
+  const int64_t per_sm = (n + num_sms() - 1) / num_sms();
+  if (per_sm <= (tau ? 16 : 8)) return 32;
+  if (least <= 16 && per_sm <= (tau ? 16 : 12)) return 16;
+  if (least <= 8 && per_sm <= 32) return 8;
+  const int most = least == 4 ? (tau ? 160 : 112)
+                   : least == 8 ? (tau ? 96 : 80)
+                   : least == 16 ? 32 : 16;
+  return per_sm <= most ? least : 0;
+}
+
 int single_run(const uint32_t* h_blob, const uint32_t* d_blob,
                const pyst_run_desc* run, const pyst_outputs* out,
                void* d_workspace, size_t workspace_bytes, void* stream,
@@ -186,6 +214,18 @@ int single_run(const uint32_t* h_blob, const uint32_t* d_blob,
     return PYST_EUNSUPPORTED;
   const uint64_t idb = (uint64_t)run->traj_id_base;
   const int64_t n = run->n_traj;
+  // (a caller that sets the sorted scheduler's geometry or asks for the
+  // simple tau loop gets the kernel it names)
+  if (mapping == PYST_MAP_THREAD &&
+      !(tau && ((run->flags & PYST_FLAG_UNSORTED) || run->round_ssa ||
+                run->round_leap || run->pool_slots || run->sorted_block))) {
+    const int lanes = group_lanes(mi, n, tau);
+    if (lanes) {
+      auto launch = tau ? (score ? launch_group_11 : launch_group_10)
+                        : (score ? launch_group_01 : launch_group_00);
+      return launch(lanes, d_blob, mi, n, idb, ra, ob, queue, st);
+    }
+  }
   if (mapping == PYST_MAP_THREAD && tau &&
       !(run->flags & PYST_FLAG_UNSORTED) && mi.nlaw == 0) {
     // (models with general kinetic laws take the simple tau loop: the
@@ -333,11 +373,12 @@ int pyst_batch_run(const uint32_t* d_blobs, const pyst_batch_item* d_items,
   if (cudaMemsetAsync(done, 0, (size_t)n_items * sizeof(uint32_t), st) !=
       cudaSuccess)
     return PYST_ECUDA;
-  if (out->score)
-    return launch_batch_1(d_blobs, d_items, n_items, lim, ra, ob, queue, done,
-                          bs, st);
-  return launch_batch_0(d_blobs, d_items, n_items, lim, ra, ob, queue, done,
-                        bs, st);
+  const bool groups = (run->flags & PYST_FLAG_LANE_GROUPS) != 0;
+  if (groups)
+    return (out->score ? launch_batch_11 : launch_batch_10)(
+        d_blobs, d_items, n_items, lim, ra, ob, queue, done, bs, st);
+  return (out->score ? launch_batch_01 : launch_batch_00)(
+      d_blobs, d_items, n_items, lim, ra, ob, queue, done, bs, st);
 }
 
 int pyst_score_backward_workspace_size(int64_t n_traj, int32_t n_reactions,

@@ -3,9 +3,11 @@
 // from a device queue (an atomic counter in caller workspace), stage the
 // item's model blob into shared memory with one bulk-async copy, and run its
 // trajectories thread-per-trajectory or warp-per-trajectory as the item
-// says.  Replaces the reference's one-JIT-and-launch-sequence-per-model
+// says (PYST_GROUPS: for batches too small to fill the GPU thread by thread,
+// a group of lanes per trajectory where the item's model allows it).  Replaces the reference's one-JIT-and-launch-sequence-per-model
 // sweep (examples/*_sim.py loops over CuTauLeaping().run, e.g.
 // examples/schlogl_sim.py:66-80).  Built once per PYST_SCORE flavour.
+#include "pyst_group.cuh"
 #include "pyst_launch.cuh"
 
 // Blocks of 128 threads per SM the register allocation must allow: 6 (at
@@ -13,7 +15,11 @@
 // Schlogl/Lotka-Volterra sweep (2048 models, scores, statistics) and 1.5%
 // slower on synthetic networks of up to 256 reactions; 0 leaves it open.
 #ifndef PYST_BATCH_MINB
+#if PYST_GROUPS
+#define PYST_BATCH_MINB 4  // as k_group
+#else
 #define PYST_BATCH_MINB 6
+#endif
 #endif
 #if PYST_BATCH_MINB > 0
 #define PYST_BATCH_BOUNDS __launch_bounds__(128, PYST_BATCH_MINB)
@@ -25,7 +31,7 @@ namespace pyst {
 // nvcc gives template functions of an anonymous namespace weak external
 // linkage on the host side, so the flavours built from this file would be
 // merged at link time; a per-flavour namespace keeps them apart.
-namespace PYST_CAT(batch_flavour_, PYST_SCORE, ) {
+namespace PYST_CAT(batch_flavour_, PYST_GROUPS, PYST_SCORE) {
 
 // Summary statistics and score Jacobians of one finished model (U
 // trajectories), computed by the block that ran it -- or, for a model split
@@ -112,16 +118,21 @@ __global__ void PYST_BATCH_BOUNDS
     k_batch(const uint32_t* __restrict__ gblobs,
             const pyst_batch_item* __restrict__ items, int64_t n_items,
             RunArgs ra, OutBase ob, unsigned long long* queue, unsigned* done,
-            int max_blob_words, int warp_bytes, int dyn_bytes, int pk_bytes) {
+            int max_blob_words, int warp_bytes, int dyn_bytes, int pk_bytes,
+            int fd_bytes, int parts, int part) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ long long s_item;
   __shared__ int s_last;
+#if PYST_GROUPS
+  __shared__ int s_next;
+#endif
   uint32_t* sblob = (uint32_t*)smem;
   uint64_t* bar = (uint64_t*)(smem + (size_t)max_blob_words * 4);
   // packed reaction descriptors of the current item (thread mapping)
   uint32_t* spk = (uint32_t*)(smem + (size_t)max_blob_words * 4 + 16);
-  unsigned char* dyn =
-      smem + (size_t)max_blob_words * 4 + 16 + (size_t)pk_bytes;
+  // and its direct forms (fd_bytes 0: the launch has no room for them)
+  uint4* sfd = (uint4*)((unsigned char*)spk + pk_bytes);
+  unsigned char* dyn = (unsigned char*)sfd + fd_bytes;
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
     fence_barrier_init();
@@ -133,12 +144,21 @@ __global__ void PYST_BATCH_BOUNDS
     if (threadIdx.x == 0) s_item = (long long)atomicAdd(queue, 1ull);
     __syncthreads();
     const long long it = s_item;
-    if (it >= n_items) break;
-    const pyst_batch_item item = items[it];
+    if (it >= n_items * parts) break;
+    pyst_batch_item item = items[PYST_GROUPS ? it / parts : it];
     // the model's trajectory count (a split model's chunks share it) and
     // this item's first trajectory in it
     const int64_t U = item.model_n_traj > 0 ? item.model_n_traj : item.n_traj;
-    const int64_t cb = item.model_n_traj > 0 ? item.chunk_begin : 0;
+    int64_t cb = item.model_n_traj > 0 ? item.chunk_begin : 0;
+    int chunks = item.group_chunks > 1 ? item.group_chunks : 1;
+    if (PYST_GROUPS && parts > 1) {
+      // this block's part of the item: a chunk of the chunk
+      const int64_t lo = (it % parts) * (int64_t)part;
+      const int64_t left = item.n_traj - lo;
+      cb += lo;
+      item.n_traj = left < 0 ? 0 : left < part ? left : part;
+      chunks *= parts;
+    }
     const uint32_t* blob = gblobs + item.blob_offset;
     const int words = (int)__ldg(blob + PYST_H_WORDS);
     const bool ok = stage_blob(sblob, blob, words, bar, parity,
@@ -173,31 +193,79 @@ __global__ void PYST_BATCH_BOUNDS
           packed_bytes(m.R) <= (size_t)pk_bytes) {
         // (uniform over the block: every thread reads the same item)
         m.pk = spk;
+        if (fd_bytes && m.nlaw == 0 &&
+            has_direct_forms(m.R, blob_direct_factors(sblob))) {
+          m.fd = sfd;
+          build_direct(m, sfd, bs);
+        }
         m.fast = __syncthreads_and(pack_reactions(m, spk)) != 0;
       }
       const bool tau = item.method == PYST_METHOD_TAU_LEAP;
+#if PYST_GROUPS
+      // (block-uniform) 4 lanes per trajectory where reactions and species
+      // allow, else 8
+      const int factors =
+          item.mapping == PYST_MAP_THREAD && m.nlaw == 0 && m.fast
+              ? blob_direct_factors(sblob) : 0;
+      const int lanes = factors < 1 || factors > 3 || m.S > 8 ? 0
+                        : m.R <= 4 && m.S <= 4 ? 4 : 8;
+      if (lanes) {
+        auto out = [&](int64_t u) {
+          return ob.at(item.sample_offset, u, item.traj_offset,
+                       item.score_offset, U, m.R);
+        };
+        // trajectories of the item in order, to the groups as they ask
+        if (threadIdx.x == 0) s_next = 0;
+        __syncthreads();
+        auto next = [&](bool first, bool want) {
+          (void)first;
+          const int lg = lanes;
+          int v = 0;
+          if (want && (threadIdx.x & (lg - 1)) == 0)
+            v = atomicAdd(&s_next, 1);
+          v = __shfl_sync(0xffffffffu, v, 0, lg);
+          return v < item.n_traj ? cb + v : cb + item.n_traj;
+        };
+        const uint64_t idb = (uint64_t)item.traj_id_base;
+        const int64_t end = cb + item.n_traj;
+        if (lanes == 4) {
+          if (tau)
+            run_groups<4, 3, 4, true, SCORE>(m, ra, idb, end, next, out);
+          else
+            run_groups<4, 3, 4, false, SCORE>(m, ra, idb, end, next, out);
+        } else {
+          if (tau)
+            run_groups<8, 3, 8, true, SCORE>(m, ra, idb, end, next, out);
+          else
+            run_groups<8, 3, 8, false, SCORE>(m, ra, idb, end, next, out);
+        }
+      } else
+#endif
       if (item.mapping == PYST_MAP_THREAD) {
         int32_t* xcol = (int32_t*)dyn + threadIdx.x;
+        const bool direct = !PYST_GROUPS && m.fast && m.fd != nullptr;
         int64_t* slot =
-            (int64_t*)((int32_t*)dyn + (size_t)m.S * bs) + threadIdx.x;
+            (int64_t*)((int32_t*)dyn + (size_t)(m.S + (direct ? 1 : 0)) * bs) +
+            threadIdx.x;
         for (int64_t v = threadIdx.x; v < item.n_traj; v += bs) {
           const int64_t u = cb + v;
           const TrajOut o = ob.at(item.sample_offset, u, item.traj_offset,
                                   item.score_offset, U, m.R);
           const uint64_t id = (uint64_t)item.traj_id_base + (uint64_t)u;
-          if (m.fast && m.R >= 2 && m.R <= 8) {
-            // (block-uniform) a packable item of 2 to 8 reactions: the
-            // reaction count fixed at compile time (the 16,384-set sweep's
-            // Lotka-Volterra and Schlogl items: 2,048 sets 3.86 -> 2.86 s)
+          if (!PYST_GROUPS && direct) {
+            // (block-uniform) an item with direct forms: the reaction count
+            // (2 to 8) fixed at compile time, three factor slots (one form
+            // for all items keeps the kernel's size)
+#if !PYST_GROUPS
             switch (m.R) {
 #define PYST_EXACT_CASE(r)                                                 \
   case r:                                                                  \
     if (tau)                                                               \
-      run_thread<r, true, SCORE, kPkPacked, r>(m, xcol, slot, bs, ra, id, \
-                                               o);                         \
+      run_thread<r, true, SCORE, kPkPacked, r, 3>(m, xcol, slot, bs, ra,   \
+                                                  id, o);                  \
     else                                                                   \
-      run_thread<r, false, SCORE, kPkPacked, r>(m, xcol, slot, bs, ra, id, \
-                                                o);                        \
+      run_thread<r, false, SCORE, kPkPacked, r, 3>(m, xcol, slot, bs, ra,  \
+                                                   id, o);                 \
     break;
               PYST_EXACT_CASE(2)
               PYST_EXACT_CASE(3)
@@ -208,6 +276,7 @@ __global__ void PYST_BATCH_BOUNDS
               PYST_EXACT_CASE(8)
 #undef PYST_EXACT_CASE
             }
+#endif
           } else if (m.R <= 8) {
             if (tau) run_thread<8, true, SCORE>(m, xcol, slot, bs, ra, id, o);
             else run_thread<8, false, SCORE>(m, xcol, slot, bs, ra, id, o);
@@ -237,14 +306,14 @@ __global__ void PYST_BATCH_BOUNDS
     if (ob.stats || ob.jac) {
       // a split model: every thread makes its outputs visible device-wide
       // before the chunk is counted (uniform branch)
-      if (item.group_chunks > 1) __threadfence();
+      if (chunks > 1) __threadfence();
       __syncthreads();  // the item's samples are all written
       bool last = true;
-      if (item.group_chunks > 1) {
+      if (chunks > 1) {
         // the block finishing the model's last chunk reduces the model
         if (threadIdx.x == 0) {
           s_last = atomicAdd(done + item.group, 1u) + 1u ==
-                   (unsigned)item.group_chunks;
+                   (unsigned)chunks;
           if (s_last) __threadfence();
         }
         __syncthreads();
@@ -257,9 +326,9 @@ __global__ void PYST_BATCH_BOUNDS
 }
 
 }  // namespace (flavour)
-using namespace PYST_CAT(batch_flavour_, PYST_SCORE, );
+using namespace PYST_CAT(batch_flavour_, PYST_GROUPS, PYST_SCORE);
 
-int PYST_CAT(launch_batch_, PYST_SCORE, )(
+int PYST_CAT(launch_batch_, PYST_GROUPS, PYST_SCORE)(
     const uint32_t* d_blobs, const pyst_batch_item* d_items, int64_t n_items,
     const pyst_batch_limits* lim, const RunArgs& ra, const OutBase& ob,
     unsigned long long* queue, unsigned* done, int bs, cudaStream_t st) {
@@ -272,8 +341,12 @@ int PYST_CAT(launch_batch_, PYST_SCORE, )(
                           ? lim->max_reactions
                           : PYST_THREAD_MAX_REACTIONS;
   const size_t pk_bytes = packed_bytes(maxr_pk);
-  const size_t smem = (size_t)lim->max_blob_words * 4 + 16 + pk_bytes + dyn;
+  size_t smem = (size_t)lim->max_blob_words * 4 + 16 + pk_bytes + dyn;
   if (smem > kMaxDynSmem) return PYST_EUNSUPPORTED;
+  // room for the direct forms and their columns' extra element, if it fits
+  const size_t fd = direct_bytes(kDirectMaxR), one = (size_t)bs * 4;
+  const size_t fd_bytes = smem + fd + one <= kMaxDynSmem ? fd : 0;
+  if (fd_bytes) smem += fd + one;
   auto kf = k_batch<(bool)PYST_SCORE>;
   const int rc = set_smem(kf, smem);
   if (rc) return rc;
@@ -283,11 +356,19 @@ int PYST_CAT(launch_batch_, PYST_SCORE, )(
   int per_sm = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kf, bs, smem);
   if (per_sm < 1) per_sm = 1;
+  int parts = 1, part = 0;
+#if PYST_GROUPS
+  if (lim->reserved >> 16 > 1 && (lim->reserved & 0xFFFF) > 0) {
+    parts = lim->reserved >> 16;
+    part = lim->reserved & 0xFFFF;
+  }
+#endif
   int64_t grid = (int64_t)num_sms() * per_sm;
-  if (grid > n_items) grid = n_items;
+  if (grid > n_items * parts) grid = n_items * parts;
   kf<<<(unsigned)grid, bs, smem, st>>>(d_blobs, d_items, n_items, ra, ob,
                                        queue, done, lim->max_blob_words,
-                                       (int)wb, (int)dyn, (int)pk_bytes);
+                                       (int)wb, (int)dyn, (int)pk_bytes,
+                                       (int)fd_bytes, parts, part);
   return cudaGetLastError() == cudaSuccess ? PYST_OK : PYST_ECUDA;
 }
 

@@ -21,7 +21,7 @@
 
 namespace pyst {
 // see pyst_k_thread.cu: per-flavour namespace, not an anonymous one
-namespace PYST_CAT(sorted_flavour_, PYST_SCORE, ) {
+namespace PYST_CAT(sorted_flavour_, PYST_SCORE, PYST_PART) {
 
 constexpr bool kScore = (bool)PYST_SCORE;
 // Largest block (threads) and the register budget: one block of
@@ -59,6 +59,7 @@ struct SortedSmem {
   uint32_t* blob;
   uint64_t* bar;
   uint32_t* pk;      // [2 * maxr] packed reaction descriptors
+  uint4* fd;         // [3 * maxr] direct forms (direct kernels only)
   int64_t* scratch;  // [S][block] leap scratch of the running threads
   double* t;         // per slot [pool * block] ...
   uint64_t* n;
@@ -67,7 +68,7 @@ struct SortedSmem {
   uint64_t* h;
   int64_t* traj;     // trajectory index, -1 for an empty slot
   double* integ;     // [MAXR][slots]
-  int32_t* x;        // [S][slots] species counts
+  int32_t* x;        // [S][slots] species counts (direct: [S + 1][slots])
   int32_t* f;
   uint32_t* leap_q;
   int32_t* ssa_left;
@@ -80,9 +81,10 @@ struct SortedSmem {
 
 __host__ __device__ inline size_t sorted_smem_bytes(int blob_words, int S,
                                                     int maxr, int pool,
-                                                    int block) {
+                                                    int block, bool direct) {
   const size_t slots = (size_t)pool * block;
   size_t b = (size_t)blob_words * 4 + 16 + packed_bytes(maxr);
+  if (direct) b += direct_bytes(maxr) + slots * 4;
   b += (size_t)S * block * 8;
   b += slots * (8 * 6 + 4 * 4);
   b += (size_t)S * slots * 4;
@@ -92,7 +94,8 @@ __host__ __device__ inline size_t sorted_smem_bytes(int blob_words, int S,
 }
 
 __device__ inline SortedSmem carve(unsigned char* p, int blob_words, int S,
-                                   int maxr, int pool, int block) {
+                                   int maxr, int pool, int block,
+                                   bool direct) {
   SortedSmem s;
   const int slots = pool * block;
   s.slots = slots;
@@ -102,6 +105,8 @@ __device__ inline SortedSmem carve(unsigned char* p, int blob_words, int S,
   p += 16;
   s.pk = (uint32_t*)p;
   p += packed_bytes(maxr);
+  s.fd = (uint4*)p;
+  if (direct) p += direct_bytes(maxr);
   s.scratch = (int64_t*)p;
   p += (size_t)S * block * 8;
   s.t = (double*)p;
@@ -119,7 +124,7 @@ __device__ inline SortedSmem carve(unsigned char* p, int blob_words, int S,
   s.integ = (double*)p;
   if (kScore) p += (size_t)maxr * slots * 8;
   s.x = (int32_t*)p;
-  p += (size_t)S * slots * 4;
+  p += (size_t)(S + (direct ? 1 : 0)) * slots * 4;
   s.f = (int32_t*)p;
   p += slots * 4;
   s.leap_q = (uint32_t*)p;
@@ -163,13 +168,13 @@ __device__ __forceinline__ void store_state(const SortedSmem& s, int p,
 }
 
 // Put trajectory u (or nothing, u >= n_traj) into slot p.
-template <int NACC>
+template <int NACC, bool ONE>
 __device__ __forceinline__ void fill_slot(const SortedSmem& s,
                                           const ModelView& m, int p,
                                           int64_t u, int64_t n_traj) {
   if (u < n_traj) {
     TState st;
-    thread_init<true>(m, s.x + p, s.slots, st);
+    thread_init<true, ONE>(m, s.x + p, s.slots, st);
     store_state(s, p, st);
     s.traj[p] = u;
     if (kScore) {
@@ -187,8 +192,8 @@ __device__ __forceinline__ void fill_slot(const SortedSmem& s,
 // NB: block size fixed at compile time, or 0 for blockDim.x.  PK:
 // kPkPacked for models whose every reaction packs (the host checks), else
 // kPkRuntime.  RX: MAXR when the model has exactly MAXR reactions (the
-// host checks), else 0.
-template <int MAXR, int NB, int PK, int RX = 0>
+// host checks), else 0.  FC: factor slots of the direct forms, or 0.
+template <int MAXR, int NB, int PK, int RX = 0, int FC = 0>
 __global__ void __launch_bounds__(kMaxBlock, kMinBlocks)
     k_tau_sorted(const uint32_t* __restrict__ gblob, int blob_words,
                  int64_t n_traj, uint64_t id_base, RunArgs ra, OutBase ob,
@@ -197,7 +202,7 @@ __global__ void __launch_bounds__(kMaxBlock, kMinBlocks)
   extern __shared__ __align__(16) unsigned char smem[];
   const int S = (int)__ldg(gblob + PYST_H_S);
   const int nb = NB ? NB : blockDim.x, nw = nb >> 5;
-  SortedSmem sm = carve(smem, blob_words, S, MAXR, pool, nb);
+  SortedSmem sm = carve(smem, blob_words, S, MAXR, pool, nb, FC > 0);
   const int slots = sm.slots, groups = pool * nw;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   if (tid == 0) {
@@ -234,13 +239,17 @@ __global__ void __launch_bounds__(kMaxBlock, kMinBlocks)
   const int R = m.R;
   if (MAXR > 0) {
     m.pk = sm.pk;
+    if (FC > 0) {
+      m.fd = sm.fd;
+      build_direct(m, sm.fd, slots);
+    }
     m.fast = __syncthreads_and(pack_reactions(m, sm.pk)) != 0;
   }
   constexpr int kAcc = (kScore && MAXR > 0) ? MAXR : 1;
   for (int k = 0; k < pool; ++k) {
     const int p = k * nb + tid;
     const int64_t u = lo + p;
-    fill_slot<kAcc>(sm, m, p, u < hi ? u : n_traj, n_traj);
+    fill_slot<kAcc, (FC > 0)>(sm, m, p, u < hi ? u : n_traj, n_traj);
   }
   const unsigned lt = (1u << lane) - 1u;
   int rot0 = 0, rot1 = 0;
@@ -358,19 +367,19 @@ __global__ void __launch_bounds__(kMaxBlock, kMinBlocks)
       // each round's code for the slot's group only (warps are uniform
       // but for the one mixed warp, which diverges across the two calls)
       if (st.flags & TS_LEAPGRP)
-        any_round<MAXR, true, kScore, PK, kGroupLeap, RX>(
+        any_round<MAXR, true, kScore, PK, kGroupLeap, RX, FC>(
             m, sm.x + p, sm.scratch + tid, slots, nb, ra,
             id_base + (uint64_t)u, st, integ, cnt, o, my_cap_ssa,
             my_cap_leap, true);
       else
-        any_round<MAXR, true, kScore, PK, kGroupSsa, RX>(
+        any_round<MAXR, true, kScore, PK, kGroupSsa, RX, FC>(
             m, sm.x + p, sm.scratch + tid, slots, nb, ra,
             id_base + (uint64_t)u, st, integ, cnt, o, my_cap_ssa,
             my_cap_leap, true);
       if (st.flags & TS_DONE) {
         thread_finish<(MAXR > 0 ? MAXR : 1), kScore>(m, sm.x + p, slots, st,
                                                      integ, cnt, o);
-        fill_slot<kAcc>(sm, m, p, qbase + (int64_t)atomicAdd(queue, 1ull),
+        fill_slot<kAcc, (FC > 0)>(sm, m, p, qbase + (int64_t)atomicAdd(queue, 1ull),
                         n_traj);
       } else {
         store_state(sm, p, st);
@@ -387,52 +396,33 @@ __global__ void __launch_bounds__(kMaxBlock, kMinBlocks)
   }
 }
 
-template <int MR>
-int launch_one(const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
-               uint64_t id_base, const RunArgs& ra, const OutBase& ob,
-               unsigned long long* queue, cudaStream_t st,
-               const SortedGeometry& g) {
-  const int maxr = MR > 0 ? MR : 1;
-  // the largest block (whole warps) up to the preferred size whose pools
-  // fit, first with the preferred slots per thread, then with one
+// Block size and slots per thread: the largest block (whole warps) up to the
+// preferred size whose pools fit, first with the preferred slots per thread,
+// then with one; false if none does.
+bool choose_geometry(const SortedGeometry& g, int words, int S, int maxr,
+                     bool direct, int* pool, int* block) {
   const int pref_block = g.block ? (g.block < kMaxBlock ? g.block : kMaxBlock)
                                  : kPrefBlock;
   const int pref_pool = g.pool ? (g.pool < kMaxPool ? g.pool : kMaxPool)
                                : kMaxPool;
   static const int kBlocks[] = {896, 768, 640, 512, 448, 384, 320, 256,
                                 224, 192, 160, 128, 96, 64};
-  int pool = 0, block = 0;
-  for (int p = pref_pool; p >= 1 && !block; --p)
+  for (int p = pref_pool; p >= 1; --p)
     for (int b : kBlocks)
       if (b <= pref_block &&
-          sorted_smem_bytes(mi.words, mi.S, maxr, p, b) <= kMaxDynSmem) {
-        pool = p;
-        block = b;
-        break;
+          sorted_smem_bytes(words, S, maxr, p, b, direct) <= kMaxDynSmem) {
+        *pool = p;
+        *block = b;
+        return true;
       }
-  if (!block) return PYST_EUNSUPPORTED;
-  const size_t smem = sorted_smem_bytes(mi.words, mi.S, maxr, pool, block);
-  // compile-time packed descriptors when every reaction packs (MAXR > 0)
-  constexpr int kPk = MR > 0 ? kPkPacked : kPkRuntime;
-  auto kf = mi.packable
-                ? (block == kMaxBlock ? k_tau_sorted<MR, kMaxBlock, kPk>
-                                      : k_tau_sorted<MR, 0, kPk>)
-                : (block == kMaxBlock ? k_tau_sorted<MR, kMaxBlock, kPkRuntime>
-                                      : k_tau_sorted<MR, 0, kPkRuntime>);
-  // a packable model with exactly MR reactions in the full-size block: the
-  // reaction count fixed at compile time (Schlogl, R = 4: 64.0 -> 57.8 ms)
-  if (MR > 0 && mi.packable && block == kMaxBlock && mi.R == MR)
-    kf = k_tau_sorted<MR, kMaxBlock, kPk, MR>;
-  // and the reaction counts between (2, 3 and 5 to 7), without scores
-  if constexpr (!kScore && (MR == 4 || MR == 8)) {
-    if (mi.packable && block == kMaxBlock) {
-      if (MR == 4 && mi.R == 2) kf = k_tau_sorted<2, kMaxBlock, kPkPacked, 2>;
-      if (MR == 4 && mi.R == 3) kf = k_tau_sorted<3, kMaxBlock, kPkPacked, 3>;
-      if (MR == 8 && mi.R == 5) kf = k_tau_sorted<5, kMaxBlock, kPkPacked, 5>;
-      if (MR == 8 && mi.R == 6) kf = k_tau_sorted<6, kMaxBlock, kPkPacked, 6>;
-      if (MR == 8 && mi.R == 7) kf = k_tau_sorted<7, kMaxBlock, kPkPacked, 7>;
-    }
-  }
+  return false;
+}
+
+template <class K>
+int launch_k(K kf, const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
+             uint64_t id_base, const RunArgs& ra, const OutBase& ob,
+             unsigned long long* queue, cudaStream_t st,
+             const SortedGeometry& g, int pool, int block, size_t smem) {
   const int rc = set_smem(kf, smem);
   if (rc) return rc;
   if (cudaMemsetAsync(queue, 0, sizeof(unsigned long long), st) !=
@@ -452,8 +442,104 @@ int launch_one(const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
   return cudaGetLastError() == cudaSuccess ? PYST_OK : PYST_ECUDA;
 }
 
+template <int MR>
+int launch_one(const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
+               uint64_t id_base, const RunArgs& ra, const OutBase& ob,
+               unsigned long long* queue, cudaStream_t st,
+               const SortedGeometry& g) {
+  const int maxr = MR > 0 ? MR : 1;
+  int pool = 0, block = 0;
+  if (!choose_geometry(g, mi.words, mi.S, maxr, false, &pool, &block))
+    return PYST_EUNSUPPORTED;
+  const size_t smem =
+      sorted_smem_bytes(mi.words, mi.S, maxr, pool, block, false);
+  // compile-time packed descriptors when every reaction packs (MAXR > 0)
+  constexpr int kPk = MR > 0 ? kPkPacked : kPkRuntime;
+  auto kf = mi.packable
+                ? (block == kMaxBlock ? k_tau_sorted<MR, kMaxBlock, kPk>
+                                      : k_tau_sorted<MR, 0, kPk>)
+                : (block == kMaxBlock ? k_tau_sorted<MR, kMaxBlock, kPkRuntime>
+                                      : k_tau_sorted<MR, 0, kPkRuntime>);
+  // a packable model with exactly MR reactions in the full-size block: the
+  // reaction count fixed at compile time (Schlogl, R = 4: 64.0 -> 57.8 ms)
+  if (MR > 8 && mi.packable && block == kMaxBlock && mi.R == MR)
+    kf = k_tau_sorted<MR, kMaxBlock, kPk, MR>;
+  return launch_k(kf, d_blob, mi, n, id_base, ra, ob, queue, st, g, pool,
+                  block, smem);
+}
+
+// A model with direct forms (2 to 8 packable reactions of at most three
+// factors): the reaction count and the factor slots fixed at compile time.
+// False when no block fits; the caller then takes launch_one.
+template <int R>
+bool launch_direct(const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
+                   uint64_t id_base, const RunArgs& ra, const OutBase& ob,
+                   unsigned long long* queue, cudaStream_t st,
+                   const SortedGeometry& g, int* rc) {
+  int pool = 0, block = 0;
+  if (!choose_geometry(g, mi.words, mi.S, R, true, &pool, &block))
+    return false;
+  const size_t smem =
+      sorted_smem_bytes(mi.words, mi.S, R, pool, block, true);
+  auto kf = mi.factors <= 2
+                ? (block == kMaxBlock
+                       ? k_tau_sorted<R, kMaxBlock, kPkPacked, R, 2>
+                       : k_tau_sorted<R, 0, kPkPacked, R, 2>)
+                : (block == kMaxBlock
+                       ? k_tau_sorted<R, kMaxBlock, kPkPacked, R, 3>
+                       : k_tau_sorted<R, 0, kPkPacked, R, 3>);
+  *rc = launch_k(kf, d_blob, mi, n, id_base, ra, ob, queue, st, g, pool,
+                 block, smem);
+  return true;
+}
+
 }  // namespace (flavour)
-using namespace PYST_CAT(sorted_flavour_, PYST_SCORE, );
+using namespace PYST_CAT(sorted_flavour_, PYST_SCORE, PYST_PART);
+
+// The instantiations are spread over several objects (PYST_PART: the models
+// of 2 to 4, 5 to 8 reactions with direct forms, up to 8 others and any
+// number, 9 to 16, 17 to 32), which compile in parallel.
+#define PYST_SORTED_ARGS                                                     \
+  const uint32_t *d_blob, const HostModelInfo &mi, int64_t n,                \
+      uint64_t id_base, const RunArgs &ra, const OutBase &ob,                \
+      unsigned long long *queue, const SortedGeometry &g, cudaStream_t st
+#define PYST_SORTED_NAME(part)                                               \
+  PYST_CAT(PYST_CAT(launch_tau_sorted_, PYST_SCORE, ), _, part)
+
+#if PYST_PART == 0 || PYST_PART == 1
+bool PYST_SORTED_NAME(PYST_PART)(PYST_SORTED_ARGS, int* rc) {
+  switch (mi.R) {
+#define PYST_CASE(r)                                                         \
+  case r:                                                                    \
+    return launch_direct<r>(d_blob, mi, n, id_base, ra, ob, queue, st, g, rc);
+#if PYST_PART == 0
+    PYST_CASE(2)
+    PYST_CASE(3)
+    PYST_CASE(4)
+#else
+    PYST_CASE(5)
+    PYST_CASE(6)
+    PYST_CASE(7)
+    PYST_CASE(8)
+#endif
+#undef PYST_CASE
+    default:
+      return false;
+  }
+}
+#elif PYST_PART == 3
+int PYST_SORTED_NAME(3)(PYST_SORTED_ARGS) {
+  return launch_one<16>(d_blob, mi, n, id_base, ra, ob, queue, st, g);
+}
+#elif PYST_PART == 4
+int PYST_SORTED_NAME(4)(PYST_SORTED_ARGS) {
+  return launch_one<32>(d_blob, mi, n, id_base, ra, ob, queue, st, g);
+}
+#else
+bool PYST_SORTED_NAME(0)(PYST_SORTED_ARGS, int* rc);
+bool PYST_SORTED_NAME(1)(PYST_SORTED_ARGS, int* rc);
+int PYST_SORTED_NAME(3)(PYST_SORTED_ARGS);
+int PYST_SORTED_NAME(4)(PYST_SORTED_ARGS);
 
 int PYST_CAT(launch_tau_sorted_, PYST_SCORE, )(
     int maxr, const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
@@ -466,11 +552,22 @@ int PYST_CAT(launch_tau_sorted_, PYST_SCORE, )(
 #else
   if (maxr > PYST_THREAD_MAX_REACTIONS) return PYST_EUNSUPPORTED;
 #endif
-  if (maxr <= 4) return launch_one<4>(d_blob, mi, n, id_base, ra, ob, queue, st, g);
-  if (maxr <= 8) return launch_one<8>(d_blob, mi, n, id_base, ra, ob, queue, st, g);
+  if (has_direct_forms(mi.R, mi.factors)) {
+    int rc = PYST_OK;
+    if (mi.R <= 4 ? PYST_SORTED_NAME(0)(d_blob, mi, n, id_base, ra, ob, queue,
+                                        g, st, &rc)
+                  : PYST_SORTED_NAME(1)(d_blob, mi, n, id_base, ra, ob, queue,
+                                        g, st, &rc))
+      return rc;
+  }
+  if (maxr <= 4)
+    return launch_one<4>(d_blob, mi, n, id_base, ra, ob, queue, st, g);
+  if (maxr <= 8)
+    return launch_one<8>(d_blob, mi, n, id_base, ra, ob, queue, st, g);
   if (maxr <= 16)
-    return launch_one<16>(d_blob, mi, n, id_base, ra, ob, queue, st, g);
-  return launch_one<32>(d_blob, mi, n, id_base, ra, ob, queue, st, g);
+    return PYST_SORTED_NAME(3)(d_blob, mi, n, id_base, ra, ob, queue, g, st);
+  return PYST_SORTED_NAME(4)(d_blob, mi, n, id_base, ra, ob, queue, g, st);
 }
+#endif
 
 }  // namespace pyst

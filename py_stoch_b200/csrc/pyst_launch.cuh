@@ -50,6 +50,7 @@ struct HostModelInfo {
   int S, R, words;
   int nlaw;       // reactions with a general kinetic law
   bool packable;  // every reaction fits the packed descriptors (no laws)
+  int factors;    // blob_direct_factors of a packable model, else 0
 };
 
 constexpr size_t kMaxDynSmem = 227 * 1024;
@@ -58,6 +59,11 @@ constexpr size_t kMaxDynSmem = 227 * 1024;
 // words, rounded up to 16 bytes.
 __host__ __device__ inline size_t packed_bytes(int R) {
   return ((size_t)R * 8 + 15) & ~(size_t)15;
+}
+
+// Shared memory of the direct forms (build_direct).
+__host__ __device__ inline size_t direct_bytes(int R) {
+  return (size_t)R * 48;
 }
 
 inline size_t host_warp_bytes(int S, int R, bool score) {
@@ -94,6 +100,19 @@ PYST_DECL_THREAD(1, 0)
 PYST_DECL_THREAD(1, 1)
 #undef PYST_DECL_THREAD
 
+// one trajectory per group of lanes; models that group_lanes accepts
+#define PYST_DECL_GROUP(T, SC)                                               \
+  int launch_group_##T##SC(int lanes, const uint32_t* d_blob,                \
+                           const HostModelInfo& mi, int64_t n,               \
+                           uint64_t id_base, const RunArgs& ra,              \
+                           const OutBase& ob, unsigned long long* queue,     \
+                           cudaStream_t st);
+PYST_DECL_GROUP(0, 0)
+PYST_DECL_GROUP(0, 1)
+PYST_DECL_GROUP(1, 0)
+PYST_DECL_GROUP(1, 1)
+#undef PYST_DECL_GROUP
+
 #define PYST_DECL_WARP(T, SC)                                                \
   int launch_plain_warp_##T##SC(const uint32_t* d_blob,                      \
                                 const HostModelInfo& mi, int64_t n,          \
@@ -106,14 +125,17 @@ PYST_DECL_WARP(1, 0)
 PYST_DECL_WARP(1, 1)
 #undef PYST_DECL_WARP
 
-#define PYST_DECL_BATCH(SC)                                                  \
-  int launch_batch_##SC(const uint32_t* d_blobs,                             \
+// (G: lane groups for thread-mapped items)
+#define PYST_DECL_BATCH(G, SC)                                               \
+  int launch_batch_##G##SC(const uint32_t* d_blobs,                          \
                         const pyst_batch_item* d_items, int64_t n_items,     \
                         const pyst_batch_limits* lim, const RunArgs& ra,     \
                         const OutBase& ob, unsigned long long* queue,       \
                         unsigned* done, int bs, cudaStream_t st);
-PYST_DECL_BATCH(0)
-PYST_DECL_BATCH(1)
+PYST_DECL_BATCH(0, 0)
+PYST_DECL_BATCH(0, 1)
+PYST_DECL_BATCH(1, 0)
+PYST_DECL_BATCH(1, 1)
 #undef PYST_DECL_BATCH
 
 // Geometry of the mode-sorted kernel: round lengths, and the preferred

@@ -27,6 +27,9 @@ struct ModelView {
   // `fast`: factors of reaction j at pk[j], net changes at pk[R + j].
   const uint32_t* pk;
   bool fast;
+  // Ready-to-use forms of small reactions (see build_direct), 3 words of 4
+  // per reaction, for the kernels compiled with factor slots.
+  const uint4* fd;
 
   __device__ __forceinline__ void load(const uint32_t* base) {
     w = base;
@@ -58,6 +61,7 @@ struct ModelView {
     t_max = __longlong_as_double((long long)tb);
     pk = nullptr;
     fast = false;
+    fd = nullptr;
   }
   __device__ __forceinline__ float rate(int j) const {
     return __uint_as_float(w[o_rate + j]);
