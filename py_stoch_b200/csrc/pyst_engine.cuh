@@ -137,47 +137,92 @@ __device__ __forceinline__ double law_ln(double a) {
 // explicitly rounded, the result rounded once to the FP32 propensity.  The
 // packer checks the programs' stacks; a malformed one gives NaN here (and
 // the trajectory the PYST_TRAJ_RATE status).  Out of line: one copy serves
-// every call site.
-static __device__ __noinline__ float eval_law(const ModelView& m, int j,
-                                              const int32_t* x, int xs) {
+// every call site.  Bound by the latency of its dependent operations: an
+// operand followed by a binary operation is applied to the top of the stack
+// at once, so that most operands are never pushed, the top of the stack and
+// the next two program words are in registers, and program, constants and
+// counts are read by their shared-memory addresses (all three are in shared
+// memory in every kernel; passing the model view by reference put two
+// dependent local-memory loads before each of them).  Saturating laws, direct
+// method, 10,007 trajectories: 17.1 -> 12.9 ms.
+__device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
+__device__ __forceinline__ double lds_f64(uint32_t addr) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(addr) : "memory");
+  return v;
+}
+// law: address of the program's first word, n its words; lawc: of the
+// constants; x, xs: of species 0's count and bytes between species.
+static __device__ __noinline__ float eval_law(uint32_t law, int n,
+                                              uint32_t lawc, uint32_t x,
+                                              uint32_t xs) {
   const double nan = __longlong_as_double(0x7ff8000000000000ll);
-  double st[8];
-  int sp = 0;
-  const int c1 = m.lawptr(j + 1);
-  for (int c = m.lawptr(j); c < c1; ++c) {
-    const uint32_t wd = m.law(c);
-    const int op = (int)(wd >> 24), arg = (int)(wd & 0xFFFFFFu);
+  double st[8];  // below the top: st[0 .. sp - 2]
+  double top = 0.0;
+  int sp = 0, c = 0;
+  uint32_t w0 = c < n ? lds_u32(law) : 0u;
+  uint32_t w1 = c + 1 < n ? lds_u32(law + 4u) : 0u;
+  auto step = [&]() {
+    ++c;
+    w0 = w1;
+    w1 = c + 1 < n ? lds_u32(law + 4u * (uint32_t)(c + 1)) : 0u;
+  };
+  while (c < n) {
+    int op = (int)(w0 >> 24);
+    const int arg = (int)(w0 & 0xFFFFFFu);
+    step();
+    double a, b;
     if (op == 1 || op == 2 || op == 16) {
       if (sp >= 8 || (op == 16 && sp < 1)) return (float)nan;
-      st[sp] = op == 1 ? (double)x[(int64_t)arg * xs]
-                       : (op == 2 ? m.lawc(arg) : st[sp - 1]);
-      ++sp;
+      double v = top;
+      if (op == 1)
+        // the exact conversion of an int, by placement in a double's fields
+        v = __dsub_rn(
+            __hiloint2double(0x43300000,
+                             (int)(lds_u32(x + (uint32_t)arg * xs) ^
+                                   0x80000000u)),
+            0x1.0p52 + 0x1.0p31);
+      else if (op == 2)
+        v = lds_f64(lawc + 8u * (uint32_t)arg);
+      const int nop = c < n ? (int)(w0 >> 24) : 0;
+      if (nop < 3 || nop > 7 || sp < 1) {
+        if (sp > 0) st[sp - 1] = top;
+        ++sp;
+        top = v;
+        continue;
+      }
+      a = top;
+      b = v;
+      op = nop;
+      step();
     } else if (op >= 3 && op <= 7) {
       if (sp < 2) return (float)nan;
-      const double b = st[--sp], a = st[sp - 1];
-      double r;
-      if (op == 3) r = __dadd_rn(a, b);
-      else if (op == 4) r = __dsub_rn(a, b);
-      else if (op == 5) r = __dmul_rn(a, b);
-      else if (op == 6) r = __ddiv_rn(a, b);
-      else r = law_idiv(a, b);
-      st[sp - 1] = r;
+      --sp;
+      b = top;
+      a = st[sp - 1];
     } else {
       if (sp < 1) return (float)nan;
-      const double a = st[sp - 1];
-      double r;
-      if (op == 8) r = -a;
-      else if (op == 10) r = law_exp(a);
-      else if (op == 11) r = law_ln(a);
-      else if (op == 12) r = __dsqrt_rn(a);
-      else if (op == 13) r = fabs(a);
-      else if (op == 14) r = floor(a);
-      else if (op == 15) r = ceil(a);
+      if (op == 8) top = -top;
+      else if (op == 10) top = law_exp(top);
+      else if (op == 11) top = law_ln(top);
+      else if (op == 12) top = __dsqrt_rn(top);
+      else if (op == 13) top = fabs(top);
+      else if (op == 14) top = floor(top);
+      else if (op == 15) top = ceil(top);
       else return (float)nan;
-      st[sp - 1] = r;
+      continue;
     }
+    if (op == 5) top = __dmul_rn(a, b);
+    else if (op == 3) top = __dadd_rn(a, b);
+    else if (op == 4) top = __dsub_rn(a, b);
+    else if (op == 6) top = __ddiv_rn(a, b);
+    else top = law_idiv(a, b);
   }
-  return sp == 1 ? __double2float_rn(st[0]) : (float)nan;
+  return sp == 1 ? __double2float_rn(top) : (float)nan;
 }
 
 // A propensity a kinetic law may return: finite and non-negative.
@@ -191,8 +236,13 @@ __device__ __forceinline__ bool valid_rate(float a) {
 template <bool LAWS = true>
 __device__ __forceinline__ float propensity(const ModelView& m, int j,
                                             const int32_t* xc, int xs) {
-  if (LAWS && m.nlaw && m.lawptr(j + 1) > m.lawptr(j))
-    return eval_law(m, j, xc, xs);
+  if (LAWS && m.nlaw) {
+    const int c0 = m.lawptr(j), n = m.lawptr(j + 1) - c0;
+    if (n > 0)
+      return eval_law(smem_u32(m.w + m.o_law + c0), n,
+                      smem_u32(m.w + m.o_lawc), smem_u32(xc),
+                      (uint32_t)xs * 4u);
+  }
   float a = m.rate(j);
   const int e1 = m.facptr(j + 1);
   for (int e = m.facptr(j); e < e1; ++e) {
