@@ -436,6 +436,52 @@ __device__ __forceinline__ float propensity_direct(const uint4* fd, int j,
   return a;
 }
 
+// ---- large networks ------------------------------------------------------
+// Beyond the register arrays every step evaluates every propensity, so the
+// chain of dependent loads per reaction (entry range, entry, count) and its
+// loops are what a step consists of.  For mass-action models whose reactions
+// have at most two reactant species of order 1 or 2, each block keeps one
+// 16-byte word per reaction:
+//   rate; per reactant species << 8 | 4 | falling << 1 | (order 2); 0: none
+// -- one load, then the counts.  Same operations in the same order.
+__device__ __forceinline__ size_t wide_bytes(int R) { return (size_t)R * 16; }
+
+// All threads of the block call this; true (per thread) when every reaction
+// this thread looked at fits.
+__device__ __forceinline__ bool build_wide(const ModelView& m, uint4* fw) {
+  bool ok = m.nlaw == 0;
+  for (int j = threadIdx.x; j < m.R; j += blockDim.x) {
+    uint32_t e2[2] = {0u, 0u};
+    const int e0 = m.facptr(j), e1 = m.facptr(j + 1);
+    if (e1 - e0 > 2) ok = false;
+    for (int e = e0; e < e1 && e < e0 + 2; ++e) {
+      const uint32_t fe = m.fac(e);
+      const int n = fac_order(fe);
+      if (n < 1 || n > 2) ok = false;
+      e2[e - e0] = (uint32_t)ent_lo(fe) << 8 | 4u |
+                   (uint32_t)fac_falling(fe) << 1 | (n == 2 ? 1u : 0u);
+    }
+    fw[j] = make_uint4(__float_as_uint(m.rate(j)), e2[0], e2[1], 0u);
+  }
+  return ok;
+}
+
+__device__ __forceinline__ float propensity_wide(const uint4 d,
+                                                 const int32_t* xc, int xs) {
+  float a = __uint_as_float(d.x);
+  if (d.y) {
+    const int x = xc[(int)(d.y >> 8) * xs];
+    a = __fmul_rn(a, (float)x);
+    if (d.y & 1u) a = __fmul_rn(a, (float)(x - (int)((d.y >> 1) & 1u)));
+  }
+  if (d.z) {
+    const int x = xc[(int)(d.z >> 8) * xs];
+    a = __fmul_rn(a, (float)x);
+    if (d.z & 1u) a = __fmul_rn(a, (float)(x - (int)((d.z >> 1) & 1u)));
+  }
+  return a;
+}
+
 // Entry q (< 2) of a packed net-change descriptor: species and delta.
 __device__ __forceinline__ int pnet_species(uint32_t d, int q) {
   return (int)((d >> (15 * q)) & 1023u);
@@ -1162,7 +1208,7 @@ __device__ __forceinline__ bool is_critical(const ModelView& m, int j,
   return false;
 }
 
-template <bool TAU>
+template <bool TAU, bool WIDE>
 __device__ void thread_round_big(const ModelView& m, int32_t* xcol,
                                  int64_t* slot, int bs, int ss,
                                  const RunArgs& ra, uint64_t traj_id,
@@ -1186,18 +1232,40 @@ __device__ void thread_round_big(const ModelView& m, int32_t* xcol,
   int ssa_left = st.ssa_left;
   uint32_t leap_q = st.leap_q;
   int n_ssa = 0, n_leap = 0;
-  auto xget = [&](int i) { return XV(i); };
+  auto prop = [&](int j) {
+    if constexpr (WIDE) return propensity_wide(m.fw[j], xcol, bs);
+    else return propensity(m, j, xcol, bs);
+  };
+  // the sum of the propensities is kept at kSegs places, so that a
+  // selection evaluates one segment again instead of half of all reactions
+  constexpr int kSegs = 8;
+  const int seg = (R + kSegs - 1) / kSegs;
 
   while (true) {
     if (n_ssa >= cap_ssa || n_leap >= cap_leap) break;
     double a0 = 0.0;
     bool bad_rate = false;
-    for (int j = 0; j < R; ++j) {
-      const float aj = propensity(m, j, xcol, bs);
-      bad_rate |= !valid_rate(aj);
-      a0 = __dadd_rn(a0, (double)aj);
+    double P[kSegs];
+    if constexpr (WIDE) {
+#pragma unroll
+      for (int s = 0; s < kSegs; ++s) {
+        const int j1 = (s + 1) * seg < R ? (s + 1) * seg : R;
+#pragma unroll 4
+        for (int j = s * seg; j < j1; ++j) a0 = add_rate(a0, prop(j));
+        P[s] = a0;
+      }
+      if (!rate_sum_usable(a0)) {
+        a0 = 0.0;  // zero, or an infinite or NaN propensity
+        for (int j = 0; j < R; ++j) a0 = __dadd_rn(a0, (double)prop(j));
+      }
+    } else {
+      for (int j = 0; j < R; ++j) {
+        const float aj = prop(j);
+        bad_rate |= !valid_rate(aj);
+        a0 = __dadd_rn(a0, (double)aj);
+      }
     }
-    if (m.nlaw && bad_rate) {
+    if (!WIDE && m.nlaw && bad_rate) {
       status = PYST_TRAJ_RATE;
       done = true;
       break;
@@ -1217,7 +1285,7 @@ __device__ void thread_round_big(const ModelView& m, int32_t* xcol,
       for (int i = 0; i < S; ++i) SL(i) = 0;
       for (int j = 0; j < R; ++j) {
         if (is_critical(m, j, xcol, bs)) continue;
-        const float aj = propensity(m, j, xcol, bs);
+        const float aj = prop(j);
         const int e1 = m.netptr(j + 1);
         for (int e = m.netptr(j); e < e1; ++e) {
           const uint32_t ne = m.net(e);
@@ -1250,7 +1318,7 @@ __device__ void thread_round_big(const ModelView& m, int32_t* xcol,
         double a0c = 0.0;
         for (int j = 0; j < R; ++j)
           if (is_critical(m, j, xcol, bs))
-            a0c = __dadd_rn(a0c, (double)propensity(m, j, xcol, bs));
+            a0c = __dadd_rn(a0c, (double)prop(j));
         double tau2 = __longlong_as_double(0x7ff0000000000000ll);
         uint4 wc = make_uint4(0, 0, 0, 0);
         if (a0c > 0.0) {
@@ -1266,7 +1334,7 @@ __device__ void thread_round_big(const ModelView& m, int32_t* xcol,
           int lastnz = -1;
           for (int j = 0; j < R; ++j) {
             if (!is_critical(m, j, xcol, bs)) continue;
-            const float aj = propensity(m, j, xcol, bs);
+            const float aj = prop(j);
             cum = __dadd_rn(cum, (double)aj);
             if (aj > 0.0f) lastnz = j;
             if (cum >= r) {
@@ -1292,7 +1360,7 @@ __device__ void thread_round_big(const ModelView& m, int32_t* xcol,
               kj = (j == kcrit) ? 1 : 0;
             } else {
               const float lam =
-                  __fmul_rn(propensity(m, j, xcol, bs), (float)tau);
+                  __fmul_rn(prop(j), (float)tau);
               const int k = poisson(lam, leap_key(rs, leap_q, j, retry));
               if (k < 0) bad = true;
               kj = k < 0 ? 0 : k;
@@ -1366,11 +1434,35 @@ __device__ void thread_round_big(const ModelView& m, int32_t* xcol,
     const double tau = __ddiv_rn(-pyst_log(u53(w.x, w.y)), a0);
     const double r = __dmul_rn(u53(w.z, w.w), a0);
     int sel = -1;
-    {
+    bool found = false;
+    if constexpr (WIDE) {
+      if (rate_sum_usable(a0)) {
+        // the first segment whose end reaches r (r <= a0, the last end),
+        // then the first reaction in it, from the sum at its start
+        int s = 0;
+        double cum = 0.0;
+#pragma unroll
+        for (int q = 0; q < kSegs - 1; ++q)
+          if (P[q] < r) {
+            s = q + 1;
+            cum = P[q];
+          }
+        const int j1 = (s + 1) * seg < R ? (s + 1) * seg : R;
+        for (int j = s * seg; j < j1; ++j) {
+          cum = add_rate(cum, prop(j));
+          if (cum >= r) {
+            sel = j;
+            break;
+          }
+        }
+        found = true;
+      }
+    }
+    if (!found) {
       double cum = 0.0;
       int lastnz = -1;
       for (int j = 0; j < R; ++j) {
-        const float aj = propensity(m, j, xcol, bs);
+        const float aj = prop(j);
         cum = __dadd_rn(cum, (double)aj);
         if (aj > 0.0f) lastnz = j;
         if (cum >= r) {
@@ -1438,8 +1530,8 @@ __device__ __forceinline__ void any_round(
     const TrajOut& o, int cap_ssa, int cap_leap, bool stop_on_switch) {
   if constexpr (MAXR == 0) {
     static_assert(!SCORE, "the large-R thread engine keeps no scores");
-    thread_round_big<TAU>(m, xcol, slot, bs, ss, ra, traj_id, st, o, cap_ssa,
-                          cap_leap, stop_on_switch);
+    thread_round_big<TAU, false>(m, xcol, slot, bs, ss, ra, traj_id, st, o,
+                                 cap_ssa, cap_leap, stop_on_switch);
   } else {
     thread_round<MAXR, TAU, SCORE, PK, 1, GROUP, RX, FC>(
         m, xcol, slot, bs, ss, ra, traj_id, st, integ, cnt, o, cap_ssa,
@@ -1453,8 +1545,12 @@ __device__ void run_thread_big(const ModelView& m, int32_t* xcol,
                                uint64_t traj_id, const TrajOut& o) {
   TState st;
   thread_init<TAU>(m, xcol, bs, st);
-  thread_round_big<TAU>(m, xcol, slot, bs, bs, ra, traj_id, st, o,
-                        0x7fffffff, 0x7fffffff, false);
+  if (m.fw)
+    thread_round_big<TAU, true>(m, xcol, slot, bs, bs, ra, traj_id, st, o,
+                                0x7fffffff, 0x7fffffff, false);
+  else
+    thread_round_big<TAU, false>(m, xcol, slot, bs, bs, ra, traj_id, st, o,
+                                 0x7fffffff, 0x7fffffff, false);
   thread_finish<1, false>(m, xcol, bs, st, nullptr, nullptr, o);
 }
 
@@ -1558,16 +1654,46 @@ __device__ void run_warp(const ModelView& m, const WarpSmem& ws,
   bool ssa_mode = !TAU;
   int ssa_left = 0;
   uint32_t leap_q = 0;
-  auto xget = [&](int i) { return ws.x[i]; };
+  // lane g holds the exponential variate and uniform of main-stream block
+  // vb + g, so the random block and logarithm of a step (500 cycles) are not
+  // on its chain; off is the next block's lane
+  uint64_t vb = 0;
+  int off = 0;
+  double e_l = 0.0, u_l = 0.0;
+  auto fill_variates = [&]() {
+    rs.n = vb + (uint64_t)lane;
+    const uint4 w = next_block(rs);
+    e_l = -pyst_log(u53(w.x, w.y));
+    u_l = u53(w.z, w.w);
+  };
+  fill_variates();
+  auto take_variates = [&](double& e, double& u) {
+    e = __shfl_sync(0xffffffffu, e_l, off);
+    u = __shfl_sync(0xffffffffu, u_l, off);
+    if (++off == 32) {
+      off = 0;
+      vb += 32;
+      fill_variates();
+    }
+  };
 
   while (true) {
     double part = 0.0;
     bool bad_rate = false;
-    for (int j = j0; j < j1; ++j) {
-      const float aj = propensity(m, j, ws.x, 1);
-      bad_rate |= !valid_rate(aj);
-      ws.a[j] = aj;
-      part = __dadd_rn(part, (double)aj);
+    if (m.fw) {  // (uniform)
+#pragma unroll 4
+      for (int j = j0; j < j1; ++j) {
+        const float aj = propensity_wide(m.fw[j], ws.x, 1);
+        ws.a[j] = aj;
+        part = __dadd_rn(part, (double)aj);
+      }
+    } else {
+      for (int j = j0; j < j1; ++j) {
+        const float aj = propensity(m, j, ws.x, 1);
+        bad_rate |= !valid_rate(aj);
+        ws.a[j] = aj;
+        part = __dadd_rn(part, (double)aj);
+      }
     }
     const double incl = warp_incl_scan(part, lane);
     const double a0 = __shfl_sync(0xffffffffu, incl, 31);
@@ -1630,16 +1756,17 @@ __device__ void run_warp(const ModelView& m, const WarpSmem& ws,
         const double inc_c = warp_incl_scan(pc, lane);
         const double a0c = __shfl_sync(0xffffffffu, inc_c, 31);
         double tau2 = __longlong_as_double(0x7ff0000000000000ll);
-        uint4 wc = make_uint4(0, 0, 0, 0);
+        double uc = 0.0;
         if (a0c > 0.0) {
-          wc = next_block(rs);
-          tau2 = __ddiv_rn(-pyst_log(u53(wc.x, wc.y)), a0c);
+          double ec;
+          take_variates(ec, uc);
+          tau2 = __ddiv_rn(ec, a0c);
         }
         const double tau1d = (double)tau1;
         double tau = (tau2 < tau1d) ? tau2 : tau1d;
         int kcrit = -1;
         if (tau1d > tau2) {
-          const double r = __dmul_rn(u53(wc.z, wc.w), a0c);
+          const double r = __dmul_rn(uc, a0c);
           kcrit = warp_select(ws.a, pc, inc_c, r, j0, j1, lane, ws.crit);
         }
         int retry = 0;
@@ -1749,9 +1876,10 @@ __device__ void run_warp(const ModelView& m, const WarpSmem& ws,
     }
     // ------------------------ one direct-method step -------------------
     steps++;
-    const uint4 w = next_block(rs);
-    const double tau = __ddiv_rn(-pyst_log(u53(w.x, w.y)), a0);
-    const double r = __dmul_rn(u53(w.z, w.w), a0);
+    double e, uu;
+    take_variates(e, uu);
+    const double tau = __ddiv_rn(e, a0);
+    const double r = __dmul_rn(uu, a0);
     const int sel = warp_select(ws.a, part, incl, r, j0, j1, lane, nullptr);
     const double tn = __dadd_rn(t, tau);
     if (SCORE) {

@@ -119,7 +119,7 @@ __global__ void PYST_BATCH_BOUNDS
             const pyst_batch_item* __restrict__ items, int64_t n_items,
             RunArgs ra, OutBase ob, unsigned long long* queue, unsigned* done,
             int max_blob_words, int warp_bytes, int dyn_bytes, int pk_bytes,
-            int fd_bytes, int parts, int part) {
+            int fd_bytes, int parts, int part, int wide_cap) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ long long s_item;
   __shared__ int s_last;
@@ -132,7 +132,9 @@ __global__ void PYST_BATCH_BOUNDS
   uint32_t* spk = (uint32_t*)(smem + (size_t)max_blob_words * 4 + 16);
   // and its direct forms (fd_bytes 0: the launch has no room for them)
   uint4* sfd = (uint4*)((unsigned char*)spk + pk_bytes);
-  unsigned char* dyn = (unsigned char*)sfd + fd_bytes;
+  // reaction words of large networks (wide_cap 0: no room for them)
+  uint4* sfw = (uint4*)((unsigned char*)sfd + fd_bytes);
+  unsigned char* dyn = (unsigned char*)sfw + wide_bytes(wide_cap);
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
     fence_barrier_init();
@@ -200,6 +202,11 @@ __global__ void PYST_BATCH_BOUNDS
         }
         m.fast = __syncthreads_and(pack_reactions(m, spk)) != 0;
       }
+      // (uniform: items beyond the register arrays, or warp-mapped)
+      if (m.nlaw == 0 && m.R <= wide_cap &&
+          (item.mapping != PYST_MAP_THREAD ||
+           m.R > PYST_THREAD_MAX_REACTIONS))
+        if (__syncthreads_and(build_wide(m, sfw))) m.fw = sfw;
       const bool tau = item.method == PYST_METHOD_TAU_LEAP;
 #if PYST_GROUPS
       // (block-uniform) 4 lanes per trajectory where reactions and species
@@ -347,6 +354,9 @@ int PYST_CAT(launch_batch_, PYST_GROUPS, PYST_SCORE)(
   const size_t fd = direct_bytes(kDirectMaxR), one = (size_t)bs * 4;
   const size_t fd_bytes = smem + fd + one <= kMaxDynSmem ? fd : 0;
   if (fd_bytes) smem += fd + one;
+  const size_t wide = (size_t)lim->max_reactions * 16;
+  const int wide_cap = smem + wide <= kMaxDynSmem ? lim->max_reactions : 0;
+  if (wide_cap) smem += wide;
   auto kf = k_batch<(bool)PYST_SCORE>;
   const int rc = set_smem(kf, smem);
   if (rc) return rc;
@@ -368,7 +378,7 @@ int PYST_CAT(launch_batch_, PYST_GROUPS, PYST_SCORE)(
   kf<<<(unsigned)grid, bs, smem, st>>>(d_blobs, d_items, n_items, ra, ob,
                                        queue, done, lim->max_blob_words,
                                        (int)wb, (int)dyn, (int)pk_bytes,
-                                       (int)fd_bytes, parts, part);
+                                       (int)fd_bytes, parts, part, wide_cap);
   return cudaGetLastError() == cudaSuccess ? PYST_OK : PYST_ECUDA;
 }
 

@@ -37,7 +37,7 @@ template <int MAXR, bool TAU, bool SCORE, int PK, int RX = 0, int FC = 0>
 __global__ void __launch_bounds__(128, PYST_THREAD_MINB)
     k_plain_thread(const uint32_t* __restrict__ gblob, int blob_words,
                    int64_t n_traj, uint64_t id_base, RunArgs ra, OutBase ob,
-                   unsigned long long* queue) {
+                   unsigned long long* queue, int wide) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint32_t* sblob = (uint32_t*)smem;
   uint64_t* bar = (uint64_t*)(smem + (size_t)blob_words * 4);
@@ -46,8 +46,11 @@ __global__ void __launch_bounds__(128, PYST_THREAD_MINB)
   const int R = (int)__ldg(gblob + PYST_H_R);
   uint32_t* pk = (uint32_t*)(smem + (size_t)blob_words * 4 + 16);
   uint4* fd = (uint4*)((unsigned char*)pk + (MAXR > 0 ? packed_bytes(R) : 0));
+  // (FC: the direct forms; large networks, `wide`: their reaction words)
   int32_t* xbase =
-      (int32_t*)((unsigned char*)fd + (FC > 0 ? direct_bytes(R) : 0));
+      (int32_t*)((unsigned char*)fd + (FC > 0 ? direct_bytes(R)
+                                       : MAXR == 0 && wide ? wide_bytes(R)
+                                                           : 0));
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
     fence_barrier_init();
@@ -78,6 +81,8 @@ __global__ void __launch_bounds__(128, PYST_THREAD_MINB)
     }
     m.fast = __syncthreads_and(pack_reactions(m, pk)) != 0;
   }
+  if (MAXR == 0 && wide)
+    if (__syncthreads_and(build_wide(m, fd))) m.fw = fd;
   int32_t* xcol = xbase + threadIdx.x;
   int64_t* slot =
       (int64_t*)(xbase + (size_t)(m.S + (FC > 0 ? 1 : 0)) * bs) + threadIdx.x;
@@ -177,7 +182,8 @@ int launch_group(const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
 template <class K>
 int launch_k(K kf, const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
              uint64_t id_base, const RunArgs& ra, const OutBase& ob, int bs,
-             cudaStream_t st, size_t smem, unsigned long long* queue) {
+             cudaStream_t st, size_t smem, unsigned long long* queue,
+             int wide = 0) {
   const int rc = set_smem(kf, smem);
   if (rc) return rc;
   int per_sm = 1;
@@ -187,7 +193,7 @@ int launch_k(K kf, const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
   const int64_t cap = (int64_t)num_sms() * per_sm;
   if (grid > cap) grid = cap;
   kf<<<(unsigned)grid, bs, smem, st>>>(d_blob, mi.words, n, id_base, ra, ob,
-                                       queue);
+                                       queue, wide);
   return cudaGetLastError() == cudaSuccess ? PYST_OK : PYST_ECUDA;
 }
 
@@ -201,7 +207,12 @@ int launch_one(const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
                                  kPkPacked>
                 : k_plain_thread<MR, (bool)PYST_TAU, (bool)PYST_SCORE,
                                  kPkLists>;
-  return launch_k(kf, d_blob, mi, n, id_base, ra, ob, bs, st, smem, queue);
+  // a large network's reaction words, if they fit
+  const bool wide = MR == 0 && mi.nlaw == 0 &&
+                    smem + (size_t)mi.R * 16 <= kMaxDynSmem;
+  if (wide) smem += (size_t)mi.R * 16;
+  return launch_k(kf, d_blob, mi, n, id_base, ra, ob, bs, st, smem, queue,
+                  wide ? 1 : 0);
 }
 
 // A packable model of 2 to 8 reactions: the reaction count fixed at compile

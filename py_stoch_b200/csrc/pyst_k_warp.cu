@@ -13,11 +13,13 @@ template <bool TAU, bool SCORE>
 __global__ void __launch_bounds__(128)
     k_plain_warp(const uint32_t* __restrict__ gblob, int blob_words,
                  int64_t n_traj, uint64_t id_base, RunArgs ra, OutBase ob,
-                 int warp_bytes, unsigned long long* queue) {
+                 int warp_bytes, unsigned long long* queue, int wide) {
   extern __shared__ __align__(16) unsigned char smem[];
   uint32_t* sblob = (uint32_t*)smem;
   uint64_t* bar = (uint64_t*)(smem + (size_t)blob_words * 4);
-  unsigned char* wbase = smem + (size_t)blob_words * 4 + 16;
+  uint4* fw = (uint4*)(smem + (size_t)blob_words * 4 + 16);
+  unsigned char* wbase = (unsigned char*)fw +
+                         (wide ? wide_bytes((int)__ldg(gblob + PYST_H_R)) : 0);
   if (threadIdx.x == 0) {
     mbar_init(bar, 1);
     fence_barrier_init();
@@ -44,6 +46,8 @@ __global__ void __launch_bounds__(128)
   }
   ModelView m;
   m.load(sblob);
+  if (wide)
+    if (__syncthreads_and(build_wide(m, fw))) m.fw = fw;
   unsigned char* mine = wbase + (size_t)wid * warp_bytes;
   const WarpSmem ws = warp_smem(mine, m.S, m.R);
   double* sacc = (double*)(mine + warp_smem_bytes(m.S, m.R));
@@ -63,8 +67,12 @@ int PYST_CAT(launch_plain_warp_, PYST_TAU, PYST_SCORE)(
     unsigned long long* queue, cudaStream_t st) {
   const int nw = bs / 32;
   const size_t wb = host_warp_bytes(mi.S, mi.R, PYST_SCORE);
-  const size_t smem = (size_t)mi.words * 4 + 16 + wb * nw;
+  size_t smem = (size_t)mi.words * 4 + 16 + wb * nw;
   if (smem > kMaxDynSmem) return PYST_EUNSUPPORTED;
+  // the reaction words, if they fit
+  const bool wide =
+      mi.nlaw == 0 && smem + (size_t)mi.R * 16 <= kMaxDynSmem;
+  if (wide) smem += (size_t)mi.R * 16;
   if (n <= 0) return PYST_OK;
   auto kf = k_plain_warp<(bool)PYST_TAU, (bool)PYST_SCORE>;
   const int rc = set_smem(kf, smem);
@@ -79,7 +87,7 @@ int PYST_CAT(launch_plain_warp_, PYST_TAU, PYST_SCORE)(
   const int64_t cap = (int64_t)num_sms() * per_sm;
   if (grid > cap) grid = cap;
   kf<<<(unsigned)grid, bs, smem, st>>>(d_blob, mi.words, n, id_base, ra, ob,
-                                       (int)wb, queue);
+                                       (int)wb, queue, wide ? 1 : 0);
   return cudaGetLastError() == cudaSuccess ? PYST_OK : PYST_ECUDA;
 }
 

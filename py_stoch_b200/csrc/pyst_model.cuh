@@ -30,6 +30,8 @@ struct ModelView {
   // Ready-to-use forms of small reactions (see build_direct), 3 words of 4
   // per reaction, for the kernels compiled with factor slots.
   const uint4* fd;
+  // One word of 4 per reaction for large networks (see build_wide), or null.
+  const uint4* fw;
 
   __device__ __forceinline__ void load(const uint32_t* base) {
     w = base;
@@ -62,6 +64,7 @@ struct ModelView {
     pk = nullptr;
     fast = false;
     fd = nullptr;
+    fw = nullptr;
   }
   __device__ __forceinline__ float rate(int j) const {
     return __uint_as_float(w[o_rate + j]);
