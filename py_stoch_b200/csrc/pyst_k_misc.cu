@@ -19,8 +19,8 @@ namespace {
 // computed; every thread then forms products, and thread j only has to add
 // up a column in trajectory order (8 cycles per addition).  Before, thread j
 // read its column from global memory with stride R inside that chain.  Sums,
-// moments, partials and the final sum at that size: 467 -> 146 us.
-// Columns are taken PYST_BWD_COLS at a time (32 KB of shared memory).
+// moments, partials and the final sum at that size: 467 -> 122 us.
+// Columns are taken PYST_BWD_COLS at a time (at most 32 KB of shared memory).
 #define PYST_BWD_COLS 16
 __device__ __forceinline__ void copy_async8(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(PYST_BWD_CHUNK)
                     const double* __restrict__ var,
                     const double* __restrict__ gmean,
                     const double* __restrict__ gvar, double* part) {
-  __shared__ double tile[PYST_BWD_CHUNK * PYST_BWD_COLS];
+  extern __shared__ __align__(16) double tile[];
   const int64_t u0 = blockIdx.x * (int64_t)PYST_BWD_CHUNK;
   const int64_t u = u0 + threadIdx.x;
   const int64_t rem = U - u0;
@@ -66,15 +66,23 @@ __global__ void __launch_bounds__(PYST_BWD_CHUNK)
         h = __dadd_rn(
             h, __dmul_rn(gvar[kf], __dsub_rn(__dmul_rn(d, d), var[kf])));
     };
-    int kf = 0;
-    for (; kf + 8 <= KF; kf += 8) {  // eight loads in flight
-      int32_t v[8];
+    // the next rows' samples are on their way while these are summed
+    constexpr int kRows = 12;
+    int32_t v[kRows], w[kRows];
+    auto load = [&](int kf, int32_t (&r)[kRows]) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = x[(int64_t)(kf + i) * U];
+      for (int i = 0; i < kRows; ++i)
+        r[i] = kf + i < KF ? x[(int64_t)(kf + i) * U] : 0;
+    };
+    load(0, v);
+    for (int kf = 0; kf < KF; kf += kRows) {
+      load(kf + kRows, w);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) add(kf + i, v[i]);
+      for (int i = 0; i < kRows; ++i)
+        if (kf + i < KF) add(kf + i, v[i]);
+#pragma unroll
+      for (int i = 0; i < kRows; ++i) v[i] = w[i];
     }
-    for (; kf < KF; ++kf) add(kf, x[(int64_t)kf * U]);
   }
   for (int j0 = 0;;) {
     copy_async_wait();
@@ -105,31 +113,34 @@ __global__ void __launch_bounds__(PYST_BWD_CHUNK)
 // ahead of the chain (4,096 rows: 8 cycles each, 17 us; reading them from
 // global memory inside the chain took several times that).  A block takes 32
 // columns.
-#define PYST_FIN_ROWS 64
+#define PYST_FIN_TILE 2048
 __global__ void __launch_bounds__(256)
     k_score_final(const double* __restrict__ part, int64_t nblk, int R,
                   int64_t U, double* grad) {
-  __shared__ double tile[2][PYST_FIN_ROWS * 32];
+  __shared__ double tile[2][PYST_FIN_TILE];
   const int j0 = blockIdx.x * 32;
   const int cols = R - j0 < 32 ? R - j0 : 32;
+  const int tile_rows = PYST_FIN_TILE / cols;
   auto fetch = [&](int64_t b0, double* t) {
     const int64_t left = nblk - b0;
-    const int rows = (int)(left < PYST_FIN_ROWS ? left : PYST_FIN_ROWS);
+    const int rows = (int)(left < tile_rows ? left : tile_rows);
     for (int i = threadIdx.x; i < rows * cols; i += 256) {
-      const int q = i / cols;
-      copy_async8(t + i, part + (b0 + q) * R + j0 + (i - q * cols));
+      const int q = cols == R ? 0 : i / cols;
+      copy_async8(t + i, cols == R ? part + b0 * R + i
+                                   : part + (b0 + q) * R + j0 +
+                                         (i - q * cols));
     }
   };
   double acc = 0.0;
   fetch(0, tile[0]);
   int cur = 0;
-  for (int64_t b0 = 0; b0 < nblk; b0 += PYST_FIN_ROWS, cur ^= 1) {
+  for (int64_t b0 = 0; b0 < nblk; b0 += tile_rows, cur ^= 1) {
     copy_async_wait();
     __syncthreads();  // this tile is in, the other one's chain is done
-    if (b0 + PYST_FIN_ROWS < nblk) fetch(b0 + PYST_FIN_ROWS, tile[cur ^ 1]);
+    if (b0 + tile_rows < nblk) fetch(b0 + tile_rows, tile[cur ^ 1]);
     if (threadIdx.x < cols) {
       const int64_t left = nblk - b0;
-      const int rows = (int)(left < PYST_FIN_ROWS ? left : PYST_FIN_ROWS);
+      const int rows = (int)(left < tile_rows ? left : tile_rows);
       const double* t = tile[cur] + threadIdx.x;
 #pragma unroll 8
       for (int q = 0; q < rows; ++q) acc = __dadd_rn(acc, t[q * cols]);
@@ -312,13 +323,20 @@ int64_t score_backward_blocks(int64_t U) {
   return (U + PYST_BWD_CHUNK - 1) / PYST_BWD_CHUNK;
 }
 
+namespace {
+size_t partial_smem(int R) {
+  return (size_t)PYST_BWD_CHUNK * (R < PYST_BWD_COLS ? R : PYST_BWD_COLS) *
+         sizeof(double);
+}
+}  // namespace
+
 int launch_score_backward(const int32_t* samples, const double* score,
                           int64_t U, int kappa, int ita, int R,
                           const double* mean, const double* var,
                           const double* gmean, const double* gvar,
                           double* part, double* grad, cudaStream_t st) {
   const int64_t nblk = score_backward_blocks(U);
-  k_score_partial<<<(unsigned)nblk, PYST_BWD_CHUNK, 0, st>>>(
+  k_score_partial<<<(unsigned)nblk, PYST_BWD_CHUNK, partial_smem(R), st>>>(
       samples, score, U, kappa, ita, R, mean, var, gmean, gvar, part);
   k_score_final<<<(R + 31) / 32, 256, 0, st>>>(part, nblk, R, U, grad);
   return cudaGetLastError() == cudaSuccess ? PYST_OK : PYST_ECUDA;
@@ -330,7 +348,7 @@ int launch_score_partials(const int32_t* samples, const double* score,
                           const double* gmean, const double* gvar,
                           double* part, cudaStream_t st) {
   const int64_t nblk = score_backward_blocks(U);
-  k_score_partial<<<(unsigned)nblk, PYST_BWD_CHUNK, 0, st>>>(
+  k_score_partial<<<(unsigned)nblk, PYST_BWD_CHUNK, partial_smem(R), st>>>(
       samples, score, U, kappa, ita, R, mean, var, gmean, gvar, part);
   return cudaGetLastError() == cudaSuccess ? PYST_OK : PYST_ECUDA;
 }
