@@ -482,6 +482,22 @@ __device__ __forceinline__ float propensity_wide(const uint4 d,
   return a;
 }
 
+// The same with selects for the tests (a missing factor is an exact factor
+// 1): for lanes that evaluate different reactions, which would diverge at
+// every test.
+__device__ __forceinline__ float propensity_wide_lanes(const uint4 d,
+                                                       const int32_t* xc) {
+  const int xa = xc[d.y >> 8], xb = xc[d.z >> 8];
+  const float fa = d.y ? (float)xa : 1.0f;
+  const float fb = d.z ? (float)xb : 1.0f;
+  const float ga = d.y & 1u ? (float)(xa - (int)((d.y >> 1) & 1u)) : 1.0f;
+  const float gb = d.z & 1u ? (float)(xb - (int)((d.z >> 1) & 1u)) : 1.0f;
+  float a = __fmul_rn(__uint_as_float(d.x), fa);
+  a = __fmul_rn(a, ga);
+  a = __fmul_rn(a, fb);
+  return __fmul_rn(a, gb);
+}
+
 // Entry q (< 2) of a packed net-change descriptor: species and delta.
 __device__ __forceinline__ int pnet_species(uint32_t d, int q) {
   return (int)((d >> (15 * q)) & 1023u);
@@ -1359,8 +1375,7 @@ __device__ void thread_round_big(const ModelView& m, int32_t* xcol,
             if (is_critical(m, j, xcol, bs)) {
               kj = (j == kcrit) ? 1 : 0;
             } else {
-              const float lam =
-                  __fmul_rn(prop(j), (float)tau);
+              const float lam = __fmul_rn(prop(j), (float)tau);
               const int k = poisson(lam, leap_key(rs, leap_q, j, retry));
               if (k < 0) bad = true;
               kj = k < 0 ? 0 : k;
@@ -1615,8 +1630,20 @@ __device__ __forceinline__ int warp_select(const float* a, double part,
   if (lane == L) {
     const double rr = __dsub_rn(r, __dsub_rn(incl, part));
     double cum = 0.0;
+    if (!mask && rate_sum_usable(part)) {
+      // the sums do not decrease, so the first that reaches rr comes after
+      // as many as are below it: no exit, the loads and sums overlap
+      int below = j0;
+#pragma unroll 4
+      for (int j = j0; j < j1; ++j) {
+        cum = add_rate(cum, a[j]);
+        below += cum < rr ? 1 : 0;
+      }
+      if (below < j1) sel = below;
+      cum = 0.0;
+    }
     int lastnz = -1;
-    for (int j = j0; j < j1; ++j) {
+    if (sel < 0) for (int j = j0; j < j1; ++j) {
       if (mask && !mask[j]) continue;
       const float aj = a[j];
       cum = __dadd_rn(cum, (double)aj);
@@ -1651,6 +1678,7 @@ __device__ void run_warp(const ModelView& m, const WarpSmem& ws,
   int status = PYST_TRAJ_DONE;
   bool fill_state = false;
   const double t_end = m.time(ita - 1);
+  double tf = m.time(0);  // next sample time (f < ita while running)
   bool ssa_mode = !TAU;
   int ssa_left = 0;
   uint32_t leap_q = 0;
@@ -1683,9 +1711,15 @@ __device__ void run_warp(const ModelView& m, const WarpSmem& ws,
     if (m.fw) {  // (uniform)
 #pragma unroll 4
       for (int j = j0; j < j1; ++j) {
-        const float aj = propensity_wide(m.fw[j], ws.x, 1);
+        const float aj = propensity_wide_lanes(m.fw[j], ws.x);
         ws.a[j] = aj;
-        part = __dadd_rn(part, (double)aj);
+        part = add_rate(part, aj);
+      }
+      // an infinite or NaN propensity: plain conversions
+      if (__any_sync(0xffffffffu, !(part < PYST_RATE_BIG))) {
+        part = 0.0;
+        for (int j = j0; j < j1; ++j)
+          part = __dadd_rn(part, (double)ws.a[j]);
       }
     } else {
       for (int j = j0; j < j1; ++j) {
@@ -1851,8 +1885,8 @@ __device__ void run_warp(const ModelView& m, const WarpSmem& ws,
               h = seq_mix(h, ((uint64_t)j << 32) | (uint32_t)ws.K[j]);
         }
         bool done = false;
-        while (tn >= m.time(f)) {
-          const double frac = __ddiv_rn(__dsub_rn(m.time(f), t), tau);
+        while (tn >= tf) {
+          const double frac = __ddiv_rn(__dsub_rn(tf, t), tau);
           for (int k = lane; k < kappa; k += 32) {
             const int i = m.out(k);
             const double inc = rint(__dmul_rn((double)ws.slot[i], frac));
@@ -1863,6 +1897,7 @@ __device__ void run_warp(const ModelView& m, const WarpSmem& ws,
             done = true;
             break;
           }
+          tf = m.time(f);
         }
         __syncwarp();
         for (int i = lane; i < S; i += 32)
@@ -1881,6 +1916,7 @@ __device__ void run_warp(const ModelView& m, const WarpSmem& ws,
     const double tau = __ddiv_rn(e, a0);
     const double r = __dmul_rn(uu, a0);
     const int sel = warp_select(ws.a, part, incl, r, j0, j1, lane, nullptr);
+    const int ne0 = m.netptr(sel), ne1 = m.netptr(sel + 1);
     const double tn = __dadd_rn(t, tau);
     if (SCORE) {
       const double dt = (tn >= t_end) ? __dsub_rn(t_end, t) : tau;
@@ -1889,29 +1925,31 @@ __device__ void run_warp(const ModelView& m, const WarpSmem& ws,
             __dadd_rn(score_acc[R + j], __dmul_rn((double)ws.a[j], dt));
     }
     bool done = false;
-    while (tn >= m.time(f)) {
-      for (int k = lane; k < kappa; k += 32)
-        store_sample(o, ita, k, f, ws.x[m.out(k)]);
-      f++;
-      if (f == ita) {
-        done = true;
-        break;
-      }
+    if (tn >= tf) {
+      do {
+        for (int k = lane; k < kappa; k += 32)
+          store_sample(o, ita, k, f, ws.x[m.out(k)]);
+        f++;
+        if (f == ita) {
+          done = true;
+          break;
+        }
+        tf = m.time(f);
+      } while (tn >= tf);
+      __syncwarp();  // the counts are read before they change
     }
     t = tn;
     if (done) break;
     bool over = false;
-    if (lane == 0) {
-      const int e1 = m.netptr(sel + 1);
-      for (int e = m.netptr(sel); e < e1; ++e) {
-        const uint32_t ne = m.net(e);
-        const int sp = ent_lo(ne);
-        const int64_t nx = (int64_t)ws.x[sp] + ent_hi_s16(ne);
-        if (nx < 0 || nx > PYST_I32MAX) over = true;
-        else ws.x[sp] = (int)nx;
-      }
-      if (SCORE) score_acc[sel] = __dadd_rn(score_acc[sel], 1.0);
+    // a reaction changes each species once: one entry per lane
+    for (int e = ne0 + lane; e < ne1; e += 32) {
+      const uint32_t ne = m.net(e);
+      const int sp = ent_lo(ne);
+      const int nx = (int)((uint32_t)ws.x[sp] + (uint32_t)ent_hi_s16(ne));
+      if (nx < 0) over = true;
+      else ws.x[sp] = nx;
     }
+    if (SCORE && lane == 0) score_acc[sel] = __dadd_rn(score_acc[sel], 1.0);
     __syncwarp();
     if (__any_sync(0xffffffffu, over)) {
       status = PYST_TRAJ_OVERFLOW;
