@@ -28,11 +28,11 @@
 // Measured (one B200, ms; before: the mode-sorted scheduler for tau-leaping,
 // a warp-wide tree of speculated steps for the direct method up to 2,368
 // trajectories, a thread each above): tau Schlogl 4,999 trajectories 20.2 ->
-// 9.0, 1,184 20.3 -> 3.9; tau Lotka-Volterra 20,011 85 -> 34.5, 1,184 75 ->
-// 18; direct Lotka-Volterra 1,024 72 -> 53, 4,999 119 -> 70; direct telegraph
-// 1,184 7.9 -> 2.2; a 64-set sweep of 256 trajectories with scores 236 -> 126.
-// A step takes 290 cycles of a lone warp (4 steps per vote), a leap about
-// 4,000; past 4 lanes x 112 trajectories per SM issue bounds it.
+// 9.0, 1,184 20.3 -> 3.9; tau Lotka-Volterra 20,011 85 -> 32, 1,184 75 -> 17;
+// direct Lotka-Volterra 1,024 72 -> 40, 4,700 119 -> 47; direct telegraph
+// 1,024 7.6 -> 1.6; a 64-set sweep of 256 trajectories with scores 236 ->
+// 125.  A step takes about 210 cycles of a lone warp, a leap about 4,000; past
+// 4 lanes x 112 trajectories per SM issue bounds it.
 //
 // Same algorithms and reference sources as pyst_engine.cuh.  Models: at most
 // 8 packable reactions (blob_direct_factors), at most LG species.
@@ -41,13 +41,18 @@
 
 namespace pyst {
 
-// direct-method steps per vote
-constexpr int kGroupSteps = 4;
-// votes of direct-method steps per round of the loop: a leap costs about as
-// much as 16 steps, so that groups in either mode wait little for the others
+// Direct-method steps per vote (at most the group's lanes).  The direct method
+// on Lotka-Volterra, 1,024 trajectories: 50.4 ms at 4 steps, 39.9 at 8, 38.9
+// at 16, but 16 lose on Schlogl, whose sample times are 25 to 90 steps apart
+// (1,700 trajectories: 9.0, 8.4, 9.0); tau-leaping's fallback rounds with
+// their samples and leaps between lose from 5 up (Schlogl 1,024: 3.9 at 4,
+// 4.4 at 10).
+constexpr int kGroupStepsDirect = 8, kGroupStepsTau = 4;
+// votes per round of the loop: a leap costs about as much as 16 steps, so
+// that groups in either mode wait little for the others
 constexpr int kGroupVotes = 4;
 
-// R: 4 or 8, at least the model's reaction count (missing reactions have
+// R: at most 8, at least the model's reaction count (missing reactions have
 // rate 0: their propensities add nothing and are never selected).  FC:
 // factor slots.  first(): this group's first trajectory, next(): the one
 // after (both called by all lanes of the warp, `want` telling whose result
@@ -56,6 +61,8 @@ template <int R, int FC, int LG, bool TAU, bool SCORE, class Next, class Out>
 __device__ void run_groups(const ModelView& m, const RunArgs& ra,
                            uint64_t id_base, int64_t n_traj, Next next,
                            Out out) {
+  constexpr int kMost = TAU ? kGroupStepsTau : kGroupStepsDirect;
+  constexpr int kGroupSteps = kMost < LG ? kMost : LG;
   static_assert(R <= LG && LG <= 32 && R <= 8 && kGroupSteps <= LG, "");
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31, gl = lane & (LG - 1);
@@ -137,7 +144,7 @@ __device__ void run_groups(const ModelView& m, const RunArgs& ra,
   int ssa_left = 0, exact = 0;
   uint32_t leap_q = 0;
   double integ = 0.0;
-  int64_t cnt = 0;
+  int cnt = 0;  // (as the thread engine's)
   int status = PYST_TRAJ_DONE;
   bool done = false, fill_state = false;
   // variates: this lane's of blocks vb + gl (c) and vb + LG + gl (n; valid
@@ -277,7 +284,7 @@ __device__ void run_groups(const ModelView& m, const RunArgs& ra,
 #pragma unroll
           for (int q = 0; q < FC; ++q) sxf[q] = xf[q];
           const double s_integ = integ;
-          const int64_t s_cnt = cnt;
+          const int s_cnt = cnt;
           double tt = t;
           bool bad = false;
           int sels[kGroupSteps];
@@ -593,7 +600,7 @@ __device__ void run_groups(const ModelView& m, const RunArgs& ra,
               int kown = 0;
 #pragma unroll
               for (int j = 0; j < R; ++j) kown = j == gl ? K[j] : kown;
-              cnt += kown;
+              cnt = (int)((uint32_t)cnt + (uint32_t)kown);
               integ = __dadd_rn(integ, __dmul_rn((double)a, tau));
             }
             while (tn >= tf) {

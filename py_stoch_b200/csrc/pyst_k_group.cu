@@ -100,16 +100,18 @@ int PYST_CAT(launch_group_, PYST_TAU, PYST_SCORE)(
   if (n <= 0) return PYST_OK;
 #define PYST_GO(r, fc) \
   return launch_lanes<r, fc>(lanes, d_blob, mi, n, id_base, ra, ob, queue, st)
-  if (mi.R <= 4) {
-    if (mi.factors == 1) PYST_GO(4, 1);
-    if (mi.factors == 2) PYST_GO(4, 2);
-    if (mi.factors == 3) PYST_GO(4, 3);
-    PYST_GO(4, 6);
-  }
-  if (mi.factors == 1) PYST_GO(8, 1);
-  if (mi.factors == 2) PYST_GO(8, 2);
-  if (mi.factors == 3) PYST_GO(8, 3);
-  PYST_GO(8, 6);
+#define PYST_GO_R(r)                  \
+  do {                                \
+    if (mi.factors == 1) PYST_GO(r, 1); \
+    if (mi.factors == 2) PYST_GO(r, 2); \
+    if (mi.factors == 3) PYST_GO(r, 3); \
+    PYST_GO(r, 6);                    \
+  } while (0)
+  if (mi.R <= 3) PYST_GO_R(3);
+  if (mi.R <= 4) PYST_GO_R(4);
+  if (mi.R <= 6) PYST_GO_R(6);
+  PYST_GO_R(8);
+#undef PYST_GO_R
 #undef PYST_GO
 }
 
