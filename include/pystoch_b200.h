@@ -141,8 +141,8 @@ typedef struct pyst_run_desc {
   int32_t flags;               /* PYST_FLAG_* bits                          */
   /* Geometry of the mode-sorted tau-leaping kernel (thread mapping); 0
    * takes the default.  Results do not depend on it, only the speed. */
-  int32_t round_ssa;           /* SSA steps per scheduling round (32)       */
-  int32_t round_leap;          /* leaps per scheduling round (3)            */
+  int32_t round_ssa;           /* SSA steps per scheduling round (100)      */
+  int32_t round_leap;          /* leaps per scheduling round (8)            */
   int32_t pool_slots;          /* trajectory slots per thread: 1 or 2 (2)   */
   int32_t sorted_block;        /* threads per block: 64..896, a multiple of
                                   32 (896; smaller when the pools do not fit

@@ -41,12 +41,16 @@ namespace {
 // the trajectory out of its SSA warp, falls within a round sets how long
 // lanes idle); with 1024-thread blocks longer rounds were slower still
 // (128 / 8 100, 256 / 16 107, 256 / 32 121, earlier kernels), and resizing
-// leap rounds to match the SSA rounds' measured time was slower too.
+// leap rounds to match the SSA rounds' measured time was slower too.  Since a
+// leap costs about ten steps (FP32 sampler, direct forms), whole fallback
+// rounds of 100 with 8 leaps are the best of six on every network tried, ms
+// against 40 / 4: Schlogl 262,144 39.0, 39.9; 60,000 20.6, 21.3;
+// Lotka-Volterra 65,536 95.7, 99.0; telegraph 65,536 13.1, 14.9.
 #ifndef PYST_CAP_SSA
-#define PYST_CAP_SSA 40
+#define PYST_CAP_SSA 100
 #endif
 #ifndef PYST_CAP_LEAP
-#define PYST_CAP_LEAP 4
+#define PYST_CAP_LEAP 8
 #endif
 constexpr int kSortedCapSsa = PYST_CAP_SSA;
 // Auto mapping of networks with more reactions than the register engine:
@@ -144,8 +148,8 @@ OutBase make_outbase(const pyst_outputs* out, int64_t n_traj) {
 // Lanes per trajectory for a run of n trajectories (pyst_group.cuh), or 0 for
 // a thread per trajectory.  More lanes shorten a step while warps are few;
 // past that they cost issue slots.  The lines, in trajectories per SM, lie
-// where the next form measured faster (148 SMs, ms; t: thread form, for
-// tau-leaping the mode-sorted scheduler):
+// where the next form measured faster (148 SMs, ms, four steps per vote; t:
+// thread form, for tau-leaping the mode-sorted scheduler):
 //   direct, Lotka-Volterra: 1,184 32: 53 16: 48; 2,368 16: 55 8: 52;
 //     4,999 8: 70 4: 68 t: 119; 9,472 4: 70 t: 121; 20,011 4: 147 t: 142;
 //   direct, telegraph (6 reactions): 592 32: 2.0 16: 2.2; 2,368 16: 2.4
