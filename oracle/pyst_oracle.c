@@ -475,6 +475,7 @@ static int select_rx(const orun* ru, int R, const float* a,
     }
   }
   if (L < 0) L = lastp;
+  if (L < 0) return -1; /* a NaN total and nothing positive */
   int j0 = L * c < R ? L * c : R;
   int j1 = j0 + c < R ? j0 + c : R;
   double rr = r - (incl[L] - part[L]);
@@ -696,7 +697,9 @@ static void one_trajectory(const omodel* m, const float* rate32,
     t = tn;
     if (done) break;
     int over = 0;
-    for (int i = 0; i < S; ++i) {
+    /* an unselected step (a NaN total and no positive propensity) counts as
+     * a step and an event, and changes nothing */
+    for (int i = 0; i < S && sel >= 0; ++i) {
       int v = m->net[(size_t)i * R + sel];
       if (v == 0) continue;
       int64_t nx = (int64_t)x[i] + v;
@@ -709,7 +712,7 @@ static void one_trajectory(const omodel* m, const float* rate32,
     }
     events++;
     h = mix(h, (uint64_t)sel);
-    cnt[sel] = cnt[sel] + 1.0;
+    if (sel >= 0) cnt[sel] = cnt[sel] + 1.0;
     if (ru->method == 1) {
       if (--ssa_left <= 0) ssa_mode = 0;
     }

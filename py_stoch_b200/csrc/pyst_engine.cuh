@@ -1045,7 +1045,7 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
           if (a[j] > 0.0f) lastnz = j;
           if (sel < 0 && cum >= rx) sel = j;
         }
-        if (sel < 0) sel = lastnz;
+        if (sel < 0) sel = lastnz;  // (-1: NaN, and nothing positive)
       }
       while (tn >= tf) {
         if (LG == 1 || g_lane == 0)
@@ -1081,7 +1081,9 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
     }
     t = tn;
     if (done) break;
-    {
+    // an unselected step (sel < 0: the total is NaN and no propensity is
+    // positive) counts as a step and an event, and changes nothing
+    if (sel >= 0) {
       // counts stay in [0, 2^31): a step outside wraps to a negative number
       bool over = false;
       if constexpr (FC > 0) {
@@ -1498,7 +1500,7 @@ __device__ void thread_round_big(const ModelView& m, int32_t* xcol,
     }
     t = tn;
     if (done) break;
-    {
+    if (sel >= 0) {  // (as thread_round's)
       const int e1 = m.netptr(sel + 1);
       bool over = false;
       for (int e = m.netptr(sel); e < e1; ++e) {
@@ -1916,7 +1918,9 @@ __device__ void run_warp(const ModelView& m, const WarpSmem& ws,
     const double tau = __ddiv_rn(e, a0);
     const double r = __dmul_rn(uu, a0);
     const int sel = warp_select(ws.a, part, incl, r, j0, j1, lane, nullptr);
-    const int ne0 = m.netptr(sel), ne1 = m.netptr(sel + 1);
+    // (an unselected step changes nothing, as in thread_round)
+    const int ne0 = sel >= 0 ? m.netptr(sel) : 0;
+    const int ne1 = sel >= 0 ? m.netptr(sel + 1) : 0;
     const double tn = __dadd_rn(t, tau);
     if (SCORE) {
       const double dt = (tn >= t_end) ? __dsub_rn(t_end, t) : tau;
@@ -1949,7 +1953,8 @@ __device__ void run_warp(const ModelView& m, const WarpSmem& ws,
       if (nx < 0) over = true;
       else ws.x[sp] = nx;
     }
-    if (SCORE && lane == 0) score_acc[sel] = __dadd_rn(score_acc[sel], 1.0);
+    if (SCORE && lane == 0 && sel >= 0)
+      score_acc[sel] = __dadd_rn(score_acc[sel], 1.0);
     __syncwarp();
     if (__any_sync(0xffffffffu, over)) {
       status = PYST_TRAJ_OVERFLOW;

@@ -409,7 +409,7 @@ __device__ void run_groups(const ModelView& m, const RunArgs& ra,
             t = tn;
             stop = done;
           }
-          if (!stop) fire(sel);
+          if (!stop && sel >= 0) fire(sel);  // (-1: as thread_round's)
           if (gany(!stop && x < 0)) {
             status = PYST_TRAJ_OVERFLOW;
             done = stop = true;
