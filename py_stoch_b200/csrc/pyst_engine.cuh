@@ -1634,12 +1634,13 @@ __device__ __forceinline__ int warp_select(const float* a, double part,
     double cum = 0.0;
     if (!mask && rate_sum_usable(part)) {
       // the sums do not decrease, so the first that reaches rr comes after
-      // as many as are below it: no exit, the loads and sums overlap
+      // as many as do not reach it: no exit, the loads and sums overlap
+      // (rr is NaN when another lane's sum is infinite or NaN: none reaches)
       int below = j0;
 #pragma unroll 4
       for (int j = j0; j < j1; ++j) {
         cum = add_rate(cum, a[j]);
-        below += cum < rr ? 1 : 0;
+        below += cum >= rr ? 0 : 1;
       }
       if (below < j1) sel = below;
       cum = 0.0;

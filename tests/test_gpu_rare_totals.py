@@ -52,6 +52,9 @@ def _model(kind, R, form='direct'):
         rx(1, {0: 1, 1: 1}, {0: 1}, 1e33)
         if R > 3:
             rx(2, {2: 1}, {1: 1}, 40.0)
+    elif kind == 'nan_apart':    # the source in another lane's reactions,
+        rx(0, {0: 1, 1: 1}, {0: 1}, 1e33)  # after one of propensity 0
+        rx(R - 1 if R < 5 else 3, {}, {2: 1}, 5.0)
     elif kind == 'inf':          # A -> A + B
         rx(0, {}, {2: 1}, 5.0)
         rx(1, {0: 1}, {0: 1, 1: 1}, 1e33)
@@ -94,7 +97,7 @@ def _compare(torch, r, o, n):
                                    rtol=T_RTOL, atol=1e-12)
 
 
-KINDS = ['nan', 'nan_last', 'nan_positive', 'inf', 'late_inf',
+KINDS = ['nan', 'nan_last', 'nan_positive', 'nan_apart', 'inf', 'late_inf',
          'late_nan', 'sum', 'subnormal']
 
 
