@@ -381,7 +381,7 @@ __device__ __forceinline__ float propensity_packed(float rate, uint32_t d,
 //              thread's column
 //   fd[3j + 1] what the second and the third factor subtract (0, 1, 2)
 //   fd[3j + 2] byte offset and change of the (up to) two species a firing
-//              changes
+//              changes; fd[3R + 2]: of none (an unselected step)
 // Slots a reaction does not use point to one extra element of the column,
 // after the S species, that holds 1 (a factor 1, a change by 0), so there is
 // nothing to test: with FC factor slots (1, 2 or 3, a template parameter: the
@@ -418,8 +418,9 @@ __host__ __device__ inline bool has_direct_forms(int R, int factors) {
 // before fd is read.
 __device__ __forceinline__ void build_direct(const ModelView& m, uint4* fd,
                                              int stride) {
+  const uint32_t one = (uint32_t)m.S * (uint32_t)stride * 4u;
+  if (threadIdx.x == 0) fd[3 * m.R + 2] = make_uint4(one, 0u, one, 0u);
   for (int j = threadIdx.x; j < m.R; j += blockDim.x) {
-    const uint32_t one = (uint32_t)m.S * (uint32_t)stride * 4u;
     uint32_t off[kDirectMaxFactors] = {one, one, one};
     uint32_t sub[kDirectMaxFactors] = {0, 0, 0};
     int n = 0;
@@ -652,6 +653,9 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
   // 8 reactions, four factors 1.80, 2.06; lists, 8 reactions 4.21, 3.57).
   constexpr bool kPrefix = MAXR <= (PK == kPkPacked ? 8 : 4);
   const int S = m.S, R = RX ? RX : m.R, ita = m.ita, kappa = m.kappa;
+  // the selection of a step that selects none (the direct forms have a
+  // reaction without changes there, so that a step needs no test)
+  const int kNone = FC > 0 ? R : -1;
   const bool pk = PK == kPkPacked || (PK == kPkRuntime && m.fast);
   // general kinetic laws: entry-list form only (a model with laws never
   // packs, and the sorted kernel's run-time form is not given such models)
@@ -1088,7 +1092,7 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
           if (a[j] > 0.0f) lastnz = j;
           if (sel < 0 && cum >= rx) sel = j;
         }
-        if (sel < 0) sel = lastnz;  // (-1: NaN, and nothing positive)
+        if (sel < 0) sel = lastnz < 0 ? kNone : lastnz;
       }
       while (tn >= tf) {
         if (LG == 1 || g_lane == 0)
@@ -1124,9 +1128,9 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
     }
     t = tn;
     if (done) break;
-    // an unselected step (sel < 0: the total is NaN and no propensity is
-    // positive) counts as a step and an event, and changes nothing
-    if (sel >= 0) {
+    // an unselected step (the total is NaN and no propensity is positive)
+    // counts as a step and an event, and changes nothing
+    if (FC > 0 || sel != kNone) {
       // counts stay in [0, 2^31): a step outside wraps to a negative number
       bool over = false;
       if constexpr (FC > 0) {
@@ -1169,7 +1173,7 @@ __device__ void thread_round(const ModelView& m, int32_t* xcol, int64_t* slot,
       }
     }
     n_ssa++;  // (completed steps: each is one event)
-    if (want_h) h = seq_mix(h, (uint64_t)sel);
+    if (want_h) h = seq_mix(h, sel == kNone ? ~0ull : (uint64_t)sel);
     if (SCORE) {
 #pragma unroll
       for (int j = 0; j < MAXR; ++j) cnt[j] += (j == sel) ? 1 : 0;

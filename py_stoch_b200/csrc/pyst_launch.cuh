@@ -61,9 +61,10 @@ __host__ __device__ inline size_t packed_bytes(int R) {
   return ((size_t)R * 8 + 15) & ~(size_t)15;
 }
 
-// Shared memory of the direct forms (build_direct).
+// Shared memory of the direct forms (build_direct): R reactions and one
+// without changes.
 __host__ __device__ inline size_t direct_bytes(int R) {
-  return (size_t)R * 48;
+  return (size_t)(R + 1) * 48;
 }
 
 inline size_t host_warp_bytes(int S, int R, bool score) {
