@@ -14,14 +14,21 @@ namespace {
 // h_u for a chunk of trajectories, then per-block partial sums
 // part[block][j] = sum_{u in chunk} h_u score[u][j] in trajectory order.
 // Bound by HBM: samples and scores are read once each (134 MB at 1,048,576
-// trajectories x 20 samples, 6 reactions).  The chunk's scores come into
-// shared memory by asynchronous copies, coalesced, while the h_u are
-// computed; every thread then forms products, and thread j only has to add
-// up a column in trajectory order (8 cycles per addition).  Before, thread j
-// read its column from global memory with stride R inside that chain.  Sums,
-// moments, partials and the final sum at that size: 467 -> 122 us.
-// Columns are taken PYST_BWD_COLS at a time (at most 32 KB of shared memory).
+// trajectories x 20 samples, 6 reactions).  Up to PYST_BWD_TILED columns the
+// chunk's scores come into shared memory by asynchronous copies, coalesced,
+// while the h_u are computed, PYST_BWD_COLS columns at a time (at most 32 KB);
+// thread j then adds up its column in trajectory order, the products off the
+// chain of additions (8 cycles each).  More columns are read from global
+// memory, a thread each: the tiles would follow one another, 16 threads at a
+// time (100,000 trajectories, us, tiles against columns: 24 reactions 46, 51;
+// 32 51, 52; 48 61, 52; 64 67, 51; all in tiles 256 reactions 337, now 76).
+// Sums, moments, partials and the final sum at 1,048,576 x 20, 6 reactions:
+// 467 us with a thread per column of global memory throughout, 122 with the
+// products formed in the tile by all threads, which are on one bank at 16
+// columns (partials and final sum alone: 6 reactions 123, now 115; 16 reactions
+// 252, now 134).
 #define PYST_BWD_COLS 16
+#define PYST_BWD_TILED 32
 __device__ __forceinline__ void copy_async8(void* dst, const void* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
                    smem_u32(dst)),
@@ -40,6 +47,7 @@ __global__ void __launch_bounds__(PYST_BWD_CHUNK)
                     const double* __restrict__ gmean,
                     const double* __restrict__ gvar, double* part) {
   extern __shared__ __align__(16) double tile[];
+  __shared__ double hs[PYST_BWD_CHUNK];
   const int64_t u0 = blockIdx.x * (int64_t)PYST_BWD_CHUNK;
   const int64_t u = u0 + threadIdx.x;
   const int64_t rem = U - u0;
@@ -53,8 +61,9 @@ __global__ void __launch_bounds__(PYST_BWD_CHUNK)
                                       : src + (int64_t)q * R + (i - q * cols));
     }
   };
+  const bool tiled = R <= PYST_BWD_TILED;
   int cols = R < PYST_BWD_COLS ? R : PYST_BWD_COLS;
-  fetch(0, cols);
+  if (tiled) fetch(0, cols);
   double h = 0.0;
   if (u < U) {
     const int KF = kappa * ita;
@@ -84,20 +93,28 @@ __global__ void __launch_bounds__(PYST_BWD_CHUNK)
       for (int i = 0; i < kRows; ++i) v[i] = w[i];
     }
   }
+  hs[threadIdx.x] = h;
+  if (!tiled) {
+    __syncthreads();
+    for (int j = threadIdx.x; j < R; j += PYST_BWD_CHUNK) {
+      const double* col = score + u0 * R + j;
+      double acc = 0.0;
+#pragma unroll 8
+      for (int q = 0; q < n; ++q)
+        acc = __dadd_rn(acc, __dmul_rn(hs[q], col[(int64_t)q * R]));
+      part[(int64_t)blockIdx.x * R + j] = acc;
+    }
+    return;
+  }
   for (int j0 = 0;;) {
     copy_async_wait();
-    __syncthreads();
-    if (threadIdx.x < n)
-      for (int c = 0; c < cols; ++c) {
-        double* t = tile + threadIdx.x * cols + c;
-        *t = __dmul_rn(h, *t);
-      }
     __syncthreads();
     if (threadIdx.x < cols) {
       const double* t = tile + threadIdx.x;
       double acc = 0.0;
-#pragma unroll 8
-      for (int q = 0; q < n; ++q) acc = __dadd_rn(acc, t[q * cols]);
+#pragma unroll 16
+      for (int q = 0; q < n; ++q)
+        acc = __dadd_rn(acc, __dmul_rn(hs[q], t[q * cols]));
       part[(int64_t)blockIdx.x * R + j0 + threadIdx.x] = acc;
     }
     j0 += cols;
@@ -325,6 +342,7 @@ int64_t score_backward_blocks(int64_t U) {
 
 namespace {
 size_t partial_smem(int R) {
+  if (R > PYST_BWD_TILED) return 0;
   return (size_t)PYST_BWD_CHUNK * (R < PYST_BWD_COLS ? R : PYST_BWD_COLS) *
          sizeof(double);
 }
