@@ -31,32 +31,9 @@ using namespace pyst;
 
 namespace {
 
-// Round lengths of the mode-sorted tau-leaping kernel: SSA steps and leaps
-// a trajectory advances between two regroupings of its block.  On the
-// Schlogl workload (262144 trajectories, 896-thread blocks, SSA fallback
-// rounds of 100 steps) 40 / 4 measured 64.3 ms a step, 20 / 2 64.5,
-// 50 / 5 64.6, 40 / 3 65.7, 60 / 6 66.1, 30 / 3 66.6, 32 / 3 68.3, 36 / 4
-// 69.2, 48 / 4 69.1, 45 / 4 70.0, 10 / 1 71.1 (a comb in the SSA length:
-// where the fallback's 100th step, and with it the DECIDE that may switch
-// the trajectory out of its SSA warp, falls within a round sets how long
-// lanes idle); with 1024-thread blocks longer rounds were slower still
-// (128 / 8 100, 256 / 16 107, 256 / 32 121, earlier kernels), and resizing
-// leap rounds to match the SSA rounds' measured time was slower too.  Since a
-// leap costs about ten steps (FP32 sampler, direct forms), whole fallback
-// rounds of 100 with 8 leaps are the best of six on every network tried, ms
-// against 40 / 4: Schlogl 262,144 39.0, 39.9; 60,000 20.6, 21.3;
-// Lotka-Volterra 65,536 95.7, 99.0; telegraph 65,536 13.1, 14.9.
-#ifndef PYST_CAP_SSA
-#define PYST_CAP_SSA 100
-#endif
-#ifndef PYST_CAP_LEAP
-#define PYST_CAP_LEAP 8
-#endif
-constexpr int kSortedCapSsa = PYST_CAP_SSA;
 // Auto mapping of networks with more reactions than the register engine:
 // warps when the run has at most this many trajectories per SM.
 constexpr int kWarpAutoPerSm = 32;
-constexpr int kSortedCapLeap = PYST_CAP_LEAP;
 
 // The factor and net-change sections of a host blob lie inside it (so the
 // packability check below reads only the blob).
@@ -235,8 +212,8 @@ int single_run(const uint32_t* h_blob, const uint32_t* d_blob,
     // (models with general kinetic laws take the simple tau loop: the
     // sorted kernel's engine carries no law evaluator)
     SortedGeometry g;
-    g.cap_ssa = run->round_ssa ? run->round_ssa : kSortedCapSsa;
-    g.cap_leap = run->round_leap ? run->round_leap : kSortedCapLeap;
+    g.cap_ssa = run->round_ssa;
+    g.cap_leap = run->round_leap;
     g.pool = run->pool_slots;
     g.block = run->sorted_block;
     const int rc =

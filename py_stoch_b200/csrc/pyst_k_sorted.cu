@@ -55,6 +55,28 @@ static_assert(kMaxPool <= 2,
 constexpr int kPrefBlock =
     PYST_SORTED_BLOCK < kMaxBlock ? PYST_SORTED_BLOCK : kMaxBlock;
 
+// Round lengths of the mode-sorted tau-leaping kernel: SSA steps and leaps
+// a trajectory advances between two regroupings of its block.  On the
+// Schlogl workload (262144 trajectories, 896-thread blocks, SSA fallback
+// rounds of 100 steps) 40 / 4 measured 64.3 ms a step, 20 / 2 64.5,
+// 50 / 5 64.6, 40 / 3 65.7, 60 / 6 66.1, 30 / 3 66.6, 32 / 3 68.3, 36 / 4
+// 69.2, 48 / 4 69.1, 45 / 4 70.0, 10 / 1 71.1 (a comb in the SSA length:
+// where the fallback's 100th step, and with it the DECIDE that may switch
+// the trajectory out of its SSA warp, falls within a round sets how long
+// lanes idle); with 1024-thread blocks longer rounds were slower still
+// (128 / 8 100, 256 / 16 107, 256 / 32 121, earlier kernels), and resizing
+// leap rounds to match the SSA rounds' measured time was slower too.
+// With direct forms a leap costs about ten steps (FP32 sampler), and whole
+// fallback rounds of 100 with 8 leaps are the better default, ms against
+// 40 / 4: Schlogl 262,144 39.0, 39.9; 60,000 20.6, 21.3; Lotka-Volterra
+// 65,536 95.7, 99.0; telegraph 65,536 13.1, 14.9; small models that only leap
+// 4 reactions, 150,000 1.39, 1.28; 8 reactions 2.58, 2.45.  Other models'
+// leaps are longer and gather in few rounds, 100 / 8 against 40 / 4: lists of
+// 4 reactions, 150,000 3.22, 2.66, of 8 7.1, 6.0; packable, 9 reactions 6.2,
+// 5.2; 16 reactions 11.1, 10.1; 400,000 30.8, 28.4.
+constexpr int kRoundSsa = 40, kRoundLeap = 4;
+constexpr int kRoundDirectSsa = 100, kRoundDirectLeap = 8;
+
 struct SortedSmem {
   uint32_t* blob;
   uint64_t* bar;
@@ -422,7 +444,8 @@ template <class K>
 int launch_k(K kf, const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
              uint64_t id_base, const RunArgs& ra, const OutBase& ob,
              unsigned long long* queue, cudaStream_t st,
-             const SortedGeometry& g, int pool, int block, size_t smem) {
+             const SortedGeometry& g, int pool, int block, size_t smem,
+             int round_ssa, int round_leap) {
   const int rc = set_smem(kf, smem);
   if (rc) return rc;
   if (cudaMemsetAsync(queue, 0, sizeof(unsigned long long), st) !=
@@ -437,7 +460,9 @@ int launch_k(K kf, const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
   const int64_t cap = (int64_t)num_sms() * per_sm;
   if (grid > cap) grid = cap;
   kf<<<(unsigned)grid, block, smem, st>>>(d_blob, mi.words, n, id_base, ra,
-                                          ob, queue, g.cap_ssa, g.cap_leap,
+                                          ob, queue,
+                                          g.cap_ssa ? g.cap_ssa : round_ssa,
+                                          g.cap_leap ? g.cap_leap : round_leap,
                                           pool);
   return cudaGetLastError() == cudaSuccess ? PYST_OK : PYST_ECUDA;
 }
@@ -478,7 +503,7 @@ int launch_one(const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
     }
   }
   return launch_k(kf, d_blob, mi, n, id_base, ra, ob, queue, st, g, pool,
-                  block, smem);
+                  block, smem, kRoundSsa, kRoundLeap);
 }
 
 // A model with direct forms (2 to 8 packable reactions of at most three
@@ -502,7 +527,7 @@ bool launch_direct(const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
                        ? k_tau_sorted<R, kMaxBlock, kPkPacked, R, 3>
                        : k_tau_sorted<R, 0, kPkPacked, R, 3>);
   *rc = launch_k(kf, d_blob, mi, n, id_base, ra, ob, queue, st, g, pool,
-                 block, smem);
+                 block, smem, kRoundDirectSsa, kRoundDirectLeap);
   return true;
 }
 
