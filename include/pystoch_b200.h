@@ -141,8 +141,11 @@ typedef struct pyst_run_desc {
   int32_t flags;               /* PYST_FLAG_* bits                          */
   /* Geometry of the mode-sorted tau-leaping kernel (thread mapping); 0
    * takes the default.  Results do not depend on it, only the speed. */
-  int32_t round_ssa;           /* SSA steps per scheduling round (100)      */
-  int32_t round_leap;          /* leaps per scheduling round (8)            */
+  int32_t round_ssa;           /* SSA steps per scheduling round (100; 40
+                                  for models of more than 8 reactions, more
+                                  than 3 factors or changes beyond the
+                                  packed forms)                             */
+  int32_t round_leap;          /* leaps per scheduling round (8; 4)         */
   int32_t pool_slots;          /* trajectory slots per thread: 1 or 2 (2)   */
   int32_t sorted_block;        /* threads per block: 64..896, a multiple of
                                   32 (896; smaller when the pools do not fit
@@ -190,6 +193,19 @@ int pyst_model_build(const pyst_model_desc* model, uint32_t* blob,
  * that overlap. */
 #define PYST_RUN_WORKSPACE_BYTES 256
 int pyst_run_workspace_size(const pyst_run_desc* run, size_t* bytes);
+
+/* The kernel a run takes (the answer of the dispatch, nothing is launched),
+ * and its lanes per trajectory; score: whether out->score will be set.
+ * GROUP: lane groups, small models in runs that do not fill the GPU; LOCKSTEP:
+ * a warp in lockstep, the smallest runs of other models; THREAD, SORTED: a
+ * thread per trajectory, alone or under the mode-sorted scheduler (which gives
+ * way to the former where a model's species leave no room for its pools);
+ * WARP: a warp per trajectory. */
+enum { PYST_KERNEL_GROUP = 1, PYST_KERNEL_LOCKSTEP = 2,
+       PYST_KERNEL_THREAD = 3, PYST_KERNEL_SORTED = 4,
+       PYST_KERNEL_WARP = 5 };
+int pyst_run_kernel(const uint32_t* h_blob, const pyst_run_desc* run,
+                    int32_t score, int32_t* kernel, int32_t* lanes);
 
 /* Direct-method SSA (Gillespie), one trajectory per thread or per warp.
  * Replaces CuGillespie.run and the forced-SSA path of CuTauLeaping.run
@@ -247,6 +263,12 @@ typedef struct pyst_batch_limits {
                         largest item's), and `group` must be set, one per
                         model, for unsplit models too                       */
 } pyst_batch_limits;
+
+/* Lanes per trajectory (4 or 8) of the model's thread-mapped items in a batch
+ * run with PYST_FLAG_LANE_GROUPS, 0 for a thread per trajectory, minus a
+ * PYST_E* code for a bad blob.  A block of 128 threads runs 128 / lanes
+ * trajectories at a time; items of that many fill the GPU best. */
+int pyst_batch_lanes(const uint32_t* h_blob);
 
 /* Workspace bytes pyst_batch_run needs for n_items items: the work-queue
  * counter and one completion counter per item (split models). */

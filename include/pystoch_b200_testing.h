@@ -43,7 +43,7 @@ int pyst_test_pipe(int32_t which, int32_t iters, int32_t blocks,
                    double* d_sink, void* stream);
 
 /* 1 if every reaction of the host blob fits the packed per-reaction
- * descriptors (the host's choice of the lane-tree kernel), 0 if not,
+ * descriptors (lane groups, direct forms and packed kernels), 0 if not,
  * minus a PYST_E* code for a bad blob. */
 int pyst_test_model_packable(const uint32_t* h_blob);
 

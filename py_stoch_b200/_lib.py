@@ -36,6 +36,8 @@ MAP_THREAD = 1
 MAP_WARP = 2
 FLAG_UNSORTED = 1
 FLAG_LANE_GROUPS = 2
+KERNEL_GROUP, KERNEL_LOCKSTEP, KERNEL_THREAD, KERNEL_SORTED, KERNEL_WARP = (
+    1, 2, 3, 4, 5)
 
 MAX_SPECIES = 1024
 MAX_REACTIONS = 4096
@@ -107,6 +109,10 @@ SIGNATURES = {
     'pyst_model_build': (C.c_int, [C.POINTER(ModelDesc), _p, C.c_int64]),
     'pyst_run_workspace_size': (C.c_int, [C.POINTER(RunDesc),
                                           C.POINTER(C.c_size_t)]),
+    'pyst_run_kernel': (C.c_int, [_p, C.POINTER(RunDesc), C.c_int32,
+                                  C.POINTER(C.c_int32),
+                                  C.POINTER(C.c_int32)]),
+    'pyst_batch_lanes': (C.c_int, [_p]),
     'pyst_ssa_direct_run': (C.c_int, [_p, _p, C.POINTER(RunDesc),
                                       C.POINTER(Outputs), _p, C.c_size_t,
                                       _p]),

@@ -149,6 +149,54 @@ int group_lanes(const HostModelInfo& mi, int64_t n, bool tau) {
   return per_sm <= most ? least : 0;
 }
 
+// The kernel a run takes (PYST_KERNEL_*), its lanes per trajectory and the
+// mapping after `auto`; the arguments have passed check_run.
+struct Route {
+  int kernel, lanes, mapping;
+};
+int choose_route(const HostModelInfo& mi, const pyst_run_desc* run, bool tau,
+                 bool score, Route* r) {
+  int mapping = run->mapping;
+  // auto: a thread per trajectory unless the species columns are large,
+  // the scores' register accumulators do not fit, or a run of a large
+  // network is too small to fill the GPU (a warp then spreads each step's
+  // reactions over 32 lanes instead of looping over them in one thread)
+  if (mapping == PYST_MAP_AUTO)
+    mapping = (mi.S <= 64 && (mi.R <= PYST_THREAD_MAX_REACTIONS ||
+                              (!score && run->n_traj > (int64_t)num_sms() *
+                                                           kWarpAutoPerSm)))
+                  ? PYST_MAP_THREAD
+                  : PYST_MAP_WARP;
+  r->mapping = mapping;
+  r->kernel = PYST_KERNEL_WARP;
+  r->lanes = 32;
+  if (mapping != PYST_MAP_THREAD) return PYST_OK;
+  // thread-mapped scores keep per-reaction accumulators in registers
+  if (score && mi.R > PYST_THREAD_MAX_REACTIONS) return PYST_EUNSUPPORTED;
+  // (a caller that sets the sorted scheduler's geometry or asks for the
+  // simple tau loop gets the kernel it names)
+  const bool simple = tau && (run->flags & PYST_FLAG_UNSORTED);
+  if (!(simple || (tau && (run->round_ssa || run->round_leap ||
+                           run->pool_slots || run->sorted_block)))) {
+    const int lanes = group_lanes(mi, run->n_traj, tau);
+    if (lanes) {
+      r->kernel = PYST_KERNEL_GROUP;
+      r->lanes = lanes;
+      return PYST_OK;
+    }
+  }
+  r->lanes = 1;
+  r->kernel = PYST_KERNEL_THREAD;
+  // (models with general kinetic laws take the simple tau loop: the sorted
+  // kernel's engine carries no law evaluator)
+  if (tau && !simple && mi.nlaw == 0) r->kernel = PYST_KERNEL_SORTED;
+  if (!tau && !score && takes_lockstep(mi.R, run->n_traj)) {
+    r->kernel = PYST_KERNEL_LOCKSTEP;
+    r->lanes = 32;
+  }
+  return PYST_OK;
+}
+
 int single_run(const uint32_t* h_blob, const uint32_t* d_blob,
                const pyst_run_desc* run, const pyst_outputs* out,
                void* d_workspace, size_t workspace_bytes, void* stream,
@@ -177,40 +225,18 @@ int single_run(const uint32_t* h_blob, const uint32_t* d_blob,
   cudaStream_t st = (cudaStream_t)stream;
   const bool tau = method == PYST_METHOD_TAU_LEAP;
   const bool score = out->score != nullptr;
-  int mapping = run->mapping;
   const int bs = run->block_size ? run->block_size : 128;
-  // auto: a thread per trajectory unless the species columns are large,
-  // the scores' register accumulators do not fit, or a run of a large
-  // network is too small to fill the GPU (a warp then spreads each step's
-  // reactions over 32 lanes instead of looping over them in one thread)
-  if (mapping == PYST_MAP_AUTO)
-    mapping = (mi.S <= 64 && (mi.R <= PYST_THREAD_MAX_REACTIONS ||
-                              (!score && run->n_traj > (int64_t)num_sms() *
-                                                           kWarpAutoPerSm)))
-                  ? PYST_MAP_THREAD
-                  : PYST_MAP_WARP;
-  // thread-mapped scores keep per-reaction accumulators in registers
-  if (mapping == PYST_MAP_THREAD && score &&
-      mi.R > PYST_THREAD_MAX_REACTIONS)
-    return PYST_EUNSUPPORTED;
+  Route route;
+  rc = choose_route(mi, run, tau, score, &route);
+  if (rc) return rc;
   const uint64_t idb = (uint64_t)run->traj_id_base;
   const int64_t n = run->n_traj;
-  // (a caller that sets the sorted scheduler's geometry or asks for the
-  // simple tau loop gets the kernel it names)
-  if (mapping == PYST_MAP_THREAD &&
-      !(tau && ((run->flags & PYST_FLAG_UNSORTED) || run->round_ssa ||
-                run->round_leap || run->pool_slots || run->sorted_block))) {
-    const int lanes = group_lanes(mi, n, tau);
-    if (lanes) {
-      auto launch = tau ? (score ? launch_group_11 : launch_group_10)
-                        : (score ? launch_group_01 : launch_group_00);
-      return launch(lanes, d_blob, mi, n, idb, ra, ob, queue, st);
-    }
+  if (route.kernel == PYST_KERNEL_GROUP) {
+    auto launch = tau ? (score ? launch_group_11 : launch_group_10)
+                      : (score ? launch_group_01 : launch_group_00);
+    return launch(route.lanes, d_blob, mi, n, idb, ra, ob, queue, st);
   }
-  if (mapping == PYST_MAP_THREAD && tau &&
-      !(run->flags & PYST_FLAG_UNSORTED) && mi.nlaw == 0) {
-    // (models with general kinetic laws take the simple tau loop: the
-    // sorted kernel's engine carries no law evaluator)
+  if (route.kernel == PYST_KERNEL_SORTED) {
     SortedGeometry g;
     g.cap_ssa = run->round_ssa;
     g.cap_leap = run->round_leap;
@@ -225,7 +251,7 @@ int single_run(const uint32_t* h_blob, const uint32_t* d_blob,
     // models with too many species fall back to the unsorted loop
     if (rc != PYST_EUNSUPPORTED) return rc;
   }
-  if (mapping == PYST_MAP_THREAD) {
+  if (route.mapping == PYST_MAP_THREAD) {
     if (tau)
       return score ? launch_plain_thread_11(mi.R, d_blob, mi, n, idb, ra, ob,
                                             bs, queue, st)
@@ -312,6 +338,31 @@ int pyst_tau_leap_run(const uint32_t* h_blob, const uint32_t* d_blob,
                       void* stream) {
   return single_run(h_blob, d_blob, run, out, d_workspace, workspace_bytes,
                     stream, PYST_METHOD_TAU_LEAP);
+}
+
+int pyst_run_kernel(const uint32_t* h_blob, const pyst_run_desc* run,
+                    int32_t score, int32_t* kernel, int32_t* lanes) {
+  if (!kernel || !lanes) return PYST_EINVAL;
+  HostModelInfo mi;
+  int rc = read_header(h_blob, &mi);
+  if (rc) return rc;
+  rc = check_run(run);
+  if (rc) return rc;
+  if (score && mi.nlaw > 0) return PYST_EUNSUPPORTED;
+  Route r;
+  rc = choose_route(mi, run, run->method == PYST_METHOD_TAU_LEAP, score != 0,
+                    &r);
+  if (rc) return rc;
+  *kernel = r.kernel;
+  *lanes = r.lanes;
+  return PYST_OK;
+}
+
+int pyst_batch_lanes(const uint32_t* h_blob) {
+  HostModelInfo mi;
+  const int rc = read_header(h_blob, &mi);
+  if (rc) return -rc;
+  return batch_lanes(mi.factors, mi.S, mi.R);
 }
 
 int pyst_batch_workspace_size(int64_t n_items, size_t* bytes) {

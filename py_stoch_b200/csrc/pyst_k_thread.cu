@@ -27,8 +27,6 @@ namespace PYST_CAT(thread_flavour_, PYST_TAU, PYST_SCORE) {
 #define PYST_THREAD_MINB 6
 #endif
 
-
-
 // PK: kPkPacked for models whose every reaction packs (the host checks),
 // kPkLists otherwise (general kinetic laws included).  RX: MAXR when the
 // model has exactly MAXR reactions (the host checks), else 0.
@@ -98,21 +96,19 @@ __global__ void __launch_bounds__(128, PYST_THREAD_MINB)
 }
 
 #if !PYST_TAU && !PYST_SCORE
-// Lane groups for runs too small to fill the GPU (direct method): each
-// trajectory is a long dependent chain of steps, so with at most a few
-// warps per SM the step latency, not issue throughput, sets the time.
-// kGroupLanes lanes share one trajectory (thread_round's LG form), which
-// takes the Philox and log work of the other steps off each step's chain.
-// Trajectory u is group u (static assignment); lane 0 of a group writes.
-// A whole warp per trajectory measured fastest (Lotka-Volterra, 1024
-// trajectories: 206.7 ms at 32 lanes, 217.1 at 16, 236.1 at 8): the warp
-// then never diverges between trajectories.
+// Lanes in lockstep for the smallest runs of models pyst_group.cuh does not
+// take (takes_lockstep): each trajectory is a long dependent chain of steps,
+// so the step latency, not issue throughput, sets the time.  kGroupLanes
+// lanes share one trajectory (thread_round's LG form), which takes the Philox
+// and log work of the other steps off each step's chain.  Trajectory u is
+// group u (static assignment); lane 0 of a group writes.  A whole warp per
+// trajectory measured fastest (Lotka-Volterra, 1024 trajectories: 206.7 ms at
+// 32 lanes, 217.1 at 16, 236.1 at 8): the warp then never diverges between
+// trajectories.
 #ifndef PYST_GROUP_LANES
 #define PYST_GROUP_LANES 32
 #endif
 constexpr int kGroupLanes = PYST_GROUP_LANES;
-// runs of at most this many trajectories per SM take the lane groups
-constexpr int kGroupMaxPerSm = 16;
 
 template <int MAXR, int LG>
 __global__ void __launch_bounds__(128)
@@ -284,12 +280,7 @@ int PYST_CAT(launch_plain_thread_, PYST_TAU, PYST_SCORE)(
   if (maxr > PYST_THREAD_MAX_REACTIONS) return PYST_EUNSUPPORTED;
 #endif
 #if !PYST_TAU && !PYST_SCORE
-  // runs too small to fill the GPU of models pyst_group.cuh does not take
-  // (general kinetic laws, large stoichiometries): at most kGroupMaxPerSm
-  // trajectories per SM, each on a whole warp (kGroupLanes = 32 lanes by
-  // default) in lockstep
-  if (maxr <= 8 && bs <= 128 && bs % kGroupLanes == 0 &&
-      n <= (int64_t)num_sms() * kGroupMaxPerSm) {
+  if (takes_lockstep(maxr, n)) {
     if (maxr <= 4)
       return launch_group<4>(d_blob, mi, n, id_base, ra, ob, bs, st, smem);
     return launch_group<8>(d_blob, mi, n, id_base, ra, ob, bs, st, smem);

@@ -67,6 +67,13 @@ __host__ __device__ inline size_t direct_bytes(int R) {
   return (size_t)(R + 1) * 48;
 }
 
+// Lanes per trajectory of a thread-mapped item in a batch with lane groups
+// (4 where reactions and species allow), or 0: a thread each.
+__host__ __device__ inline int batch_lanes(int factors, int S, int R) {
+  if (factors < 1 || factors > 3 || S > 8) return 0;
+  return R <= 4 && S <= 4 ? 4 : 8;
+}
+
 inline size_t host_warp_bytes(int S, int R, bool score) {
   size_t b = (size_t)S * 8 + (size_t)S * 4 + (size_t)R * 4 + (size_t)R * 4 +
              (((size_t)R + 3) & ~(size_t)3);
@@ -87,6 +94,14 @@ inline int set_smem(K kernel, size_t bytes) {
 }
 
 int num_sms();
+
+// Runs too small to fill the GPU of models pyst_group.cuh does not take
+// (general kinetic laws, large stoichiometries), direct method without
+// scores: at most 16 trajectories per SM, each on a whole warp in lockstep.
+constexpr int kLockstepMaxPerSm = 16;
+inline bool takes_lockstep(int R, int64_t n) {
+  return R <= 8 && n <= (int64_t)num_sms() * kLockstepMaxPerSm;
+}
 
 // plain, one trajectory per thread (maxr = R; picks MAXR in {4,8,16,32})
 #define PYST_DECL_THREAD(T, SC)                                              \
