@@ -257,11 +257,7 @@ typedef struct pyst_batch_limits {
   int32_t max_blob_words;
   int32_t max_species;
   int32_t max_reactions;
-  int32_t reserved;  /* 0; with PYST_FLAG_LANE_GROUPS may be parts << 16 |
-                        part: blocks then share each item in `parts` parts of
-                        `part` trajectories (parts * part at least the
-                        largest item's), and `group` must be set, one per
-                        model, for unsplit models too                       */
+  int32_t reserved;
 } pyst_batch_limits;
 
 /* Lanes per trajectory (4 or 8) of the model's thread-mapped items in a batch

@@ -22,6 +22,9 @@ from .simulator import DEFAULT_STEP_BUDGET, _mapping, _method, _torch
 
 # Resident threads per SM of the batched kernel (6 blocks of 128).
 BATCH_THREADS_PER_SM = 768
+# Threads per block of a batch with lane groups, the first that leaves few of
+# its groups without a trajectory (Batch._group_block).
+GROUP_BLOCKS = (128, 64, 32)
 
 
 def estimated_cost(model, method):
@@ -53,10 +56,17 @@ def auto_mapping(model, score=False):
 
 
 def small_model(model):
-    """Models of the size the lane groups take (the kernel checks the
+    """Models of the size the lane groups take (group_lanes looks at the
     reactions themselves)."""
     return (model.n_reactions <= 8 and model.n_species <= 8 and
             not getattr(model, 'has_laws', False))
+
+
+def group_lanes(model, blob):
+    """Lanes per trajectory of a thread-mapped model in a run with lane
+    groups, 0 if it has a thread per trajectory there too."""
+    return max(int(_lib.lib().pyst_batch_lanes(blob.ctypes.data)), 0) \
+        if small_model(model) else 0
 
 
 class Batch(object):
@@ -112,12 +122,12 @@ class Batch(object):
                                         _lib.THREAD_MAX_REACTIONS) else x
                       for m, x in zip(self.models, mp)]
         self.mappings = np.array(mp, np.int32)
+        blobs = [m.blob() for m in self.models]
         self.lane_groups = bool(chunk) and self._use_lane_groups(torch)
         if traj_id_base is None:
             traj_id_base = np.concatenate([[0], np.cumsum(self.n_traj)[:-1]])
         self.traj_id_base = np.asarray(traj_id_base, np.int64)
 
-        blobs = [m.blob() for m in self.models]
         self.blob_offset = np.concatenate(
             [[0], np.cumsum([len(b) for b in blobs])[:-1]]).astype(np.int64)
         self.kappa = np.array([m.kappa for m in self.models], np.int64)
@@ -149,55 +159,40 @@ class Batch(object):
         # thread-mapped block's trajectories per pass) is split into chunks
         # that different blocks run at once, so a few large models still
         # fill the GPU and the longest ones do not form the tail alone.
-        spans = []
-        for i in self.run_order:
-            U = int(self.n_traj[i])
-            cs = int(chunk) if chunk else 0
-            if self.mappings[i] == _lib.MAP_WARP:
-                cs = max(cs // 8, 4) if cs else 0
-            if cs and U > cs:
-                k = -(-U // cs)
-                spans += [(i, c * cs, min(cs, U - c * cs), U, k)
-                          for c in range(k)]
-            else:
-                spans.append((i, 0, U, 0, 0))
-        self.n_items = len(spans)
-        self.item_model = np.array([sp[0] for sp in spans], np.int64)
-        self.item_n_traj = np.array([sp[2] for sp in spans], np.int64)
-        items = (_lib.BatchItem * len(spans))()
-        for slot, (i, c0, cn, U, k) in enumerate(spans):
-            it = items[slot]
-            it.blob_offset = int(self.blob_offset[i])
-            it.n_traj = cn
-            it.traj_id_base = int(self.traj_id_base[i])
-            it.sample_offset = int(self.sample_offset[i])
-            it.traj_offset = int(self.traj_offset[i])
-            it.score_offset = int(self.score_offset[i])
-            it.stats_offset = int(self.stats_offset[i])
-            it.jac_offset = int(self.jac_offset[i])
-            it.method = int(self.methods[i])
-            it.mapping = int(self.mappings[i])
-            it.chunk_begin = c0
-            it.model_n_traj = U
-            it.group = int(i)
-            it.group_chunks = k
-        raw = np.frombuffer(bytes(items), dtype=np.uint8)
-        self.d_items = torch.from_numpy(raw.copy()).to(self.device)
+        size = np.full(n, int(chunk) if chunk else 0, np.int64)
+        size[self.mappings == _lib.MAP_WARP] = max(int(chunk) // 8, 4) \
+            if chunk else 0
+        items = self._items(size)
+        self.n_items = len(items)
+        self.item_model = items['group'].astype(np.int64)
+        self.item_n_traj = items['n_traj'].copy()
+        self.d_items = self._upload(torch, items)
+        # With lane groups, runs take a table whose items are one trajectory
+        # per group of a block (None: too few of the models' reactions fit).
+        self._group_items, self._n_group_items = None, 0
+        if self.lane_groups:
+            lanes = np.array(
+                [group_lanes(m, b) if x == _lib.MAP_THREAD else 0
+                 for m, b, x in zip(self.models, blobs, self.mappings)],
+                np.int64)
+            g = lanes > 0
+            if g.any() and (2 * int(self.n_traj[g].sum()) >=
+                            self.total_traj):
+                self._group_block = self._choose_block(lanes)
+                size[g] = np.minimum(size[g], self._group_block // lanes[g])
+                items = self._items(size)
+                self._group_items = self._upload(torch, items)
+                self._n_group_items = len(items)
         self.d_blobs = torch.from_numpy(
             np.concatenate(blobs).view(np.int32)).to(self.device)
         self.limits = _lib.BatchLimits(
             max(len(b) for b in blobs),
             max(m.n_species for m in self.models),
             max(m.n_reactions for m in self.models), 0)
-        if self.lane_groups:
-            # blocks share an item in parts of one trajectory per group
-            part = 32 if all(m.n_reactions <= 4 and m.n_species <= 4
-                             for m in self.models) else 16
-            parts = -(-int(self.item_n_traj.max(initial=1)) // part)
-            self.limits.reserved = min(parts, 0x7FFF) << 16 | part
         L = _lib.lib()
         ws = C.c_size_t(0)
-        _lib.check(L.pyst_batch_workspace_size(self.n_items, C.byref(ws)),
+        _lib.check(L.pyst_batch_workspace_size(
+            max(self.n_items, self._n_group_items), C.byref(ws)),
                    'pyst_batch_workspace_size')
         self.workspace = torch.empty(int(ws.value), dtype=torch.uint8,
                                      device=self.device)
@@ -228,12 +223,66 @@ class Batch(object):
                 int((2 * self.kappa * self.ita * self.R).sum()),
                 dtype=torch.float64, device=dev)
 
+    def _items(self, size):
+        """The item table: models in run order, those of more than size[i]
+        trajectories (0: any) in chunks of that many."""
+        n_traj = self.n_traj
+        split = (size > 0) & (n_traj > size)
+        parts = np.ones(len(n_traj), np.int64)
+        parts[split] = -(-n_traj[split] // size[split])
+        k = parts[self.run_order]
+        i = np.repeat(self.run_order, k)
+        at = np.arange(len(i)) - np.repeat(np.cumsum(k) - k, k)
+        split = split[i]
+        items = np.zeros(len(i), np.dtype(_lib.BatchItem))
+        for name in ('blob_offset', 'traj_id_base', 'sample_offset',
+                     'traj_offset', 'score_offset', 'stats_offset',
+                     'jac_offset'):
+            items[name] = getattr(self, name)[i]
+        items['method'] = self.methods[i]
+        items['mapping'] = self.mappings[i]
+        items['chunk_begin'] = begin = np.where(split, at * size[i], 0)
+        items['n_traj'] = np.where(
+            split, np.minimum(size[i], n_traj[i] - begin), n_traj[i])
+        items['model_n_traj'] = np.where(split, n_traj[i], 0)
+        items['group'] = i
+        items['group_chunks'] = np.where(split, k.repeat(k), 0)
+        return items
+
+    def _upload(self, torch, items):
+        return torch.from_numpy(items.view(np.uint8).copy()).to(self.device)
+
+    def _choose_block(self, lanes):
+        """Threads per block with lane groups: the largest of GROUP_BLOCKS
+        that leaves at most an eighth of its groups without a trajectory, so
+        that models of few trajectories fill their blocks; at least the
+        thread form's size where other models run beside.  Measured at 100
+        trajectories per SM (128, 64, 32 threads, ms; 8 trajectories a model:
+        Schlogl tau 5.2, 3.9, 3.1; Lotka-Volterra direct 4.5, 2.8, 1.9;
+        telegraph tau 3.7, 3.0, 2.9; 40: 3.2, 3.2, 3.0; 3.1, 1.9, 1.9; 2.8,
+        2.6, 2.7; 256: 2.8, 3.0, 2.9; 2.0, 2.0, 2.1; 2.7, 2.6, 2.6)."""
+        g = lanes > 0
+        n = self.n_traj[g]
+        least = 0 if g.all() else (
+            64 if int(self.item_n_traj.max(initial=0)) <= 64 else 128)
+        for block in GROUP_BLOCKS:
+            per = block // lanes[g]
+            if 8 * int((-(-n // per) * per - n).sum()) <= int(n.sum()):
+                break
+        return max(block, least)
+
     def _use_lane_groups(self, torch):
-        """Whether thread-mapped items run a lane group per trajectory: the
-        batch is far from filling the GPU thread by thread and at least half
-        of its trajectories are of models the lane groups take.  The lines
-        (trajectories per SM) are where the two forms meet: tau-leaping at
-        about 200, the direct method at about 96."""
+        """Whether thread-mapped items may run a lane group per trajectory:
+        the batch is far from filling the GPU thread by thread and at least
+        half of its trajectories are of models of the size the lane groups
+        take.  The lines (trajectories per SM) lie where the thread form comes
+        near (thread form against lane groups, 256 trajectories a model with
+        scores and statistics, ms): tau-leaping at 200, Schlogl 12.2, 4.8;
+        Lotka-Volterra 2.2, 1.6; telegraph 5.4, 4.5; 8 reactions 1.9, 1.8;
+        at 280 13.7, 6.1; 2.2, 1.9; 5.9, 5.9; 2.2, 2.3; the direct method at
+        100 2.8, 2.1; 2.4, 2.0; 2.3, 2.0; 1.2, 0.9; at 150 3.2, 2.7; 2.8,
+        2.8; 2.6, 2.6; 1.5, 1.2; at 200 3.2, 3.4; 2.8, 3.4; 2.7, 3.4; 1.6,
+        1.6.  (Models of 8 trajectories gain twice as much.)"""
         ok = np.array([x == _lib.MAP_THREAD and small_model(m)
                        for m, x in zip(self.models, self.mappings)], bool)
         total = int(self.n_traj.sum())
@@ -248,11 +297,14 @@ class Batch(object):
             max_leap_retries=63, step_budget=None, block_size=0):
         """Enqueue the whole batch on ``stream`` (one kernel launch).
         ``block_size`` 0 picks 64 threads when no work item has more than 64
-        trajectories (one block then covers an item), else 128."""
+        trajectories (one block then covers an item), else 128; with lane
+        groups the size their items were made for."""
         torch = _torch()
         L = _lib.lib()
+        groups = self.lane_groups and self._group_items is not None
         if not block_size:
-            block_size = 128 if self.lane_groups else 64 if int(self.item_n_traj.max()) <= 64 else 128
+            block_size = self._group_block if groups else (
+                64 if int(self.item_n_traj.max()) <= 64 else 128)
         if step_budget is None:
             step_budget = DEFAULT_STEP_BUDGET
         o = self.out
@@ -268,13 +320,14 @@ class Batch(object):
         r = _lib.RunDesc(0, 0, int(seed) & 0xFFFFFFFFFFFFFFFF, 0, 0,
                          int(ssa_fallback_steps), int(max_leap_retries),
                          int(step_budget), int(block_size),
-                         _lib.FLAG_LANE_GROUPS if self.lane_groups else 0)
+                         _lib.FLAG_LANE_GROUPS if groups else 0)
         if stream is None:
             stream = torch.cuda.current_stream(self.device)
         _lib.check(L.pyst_batch_run(
-            self.d_blobs.data_ptr(), self.d_items.data_ptr(),
-            self.n_items, C.byref(self.limits), C.byref(r),
-            C.byref(outs), self.workspace.data_ptr(),
+            self.d_blobs.data_ptr(),
+            (self._group_items if groups else self.d_items).data_ptr(),
+            self._n_group_items if groups else self.n_items,
+            C.byref(self.limits), C.byref(r), C.byref(outs), self.workspace.data_ptr(),
             self.workspace.numel(), C.c_void_p(stream.cuda_stream)),
             'pyst_batch_run')
         return self

@@ -4,9 +4,11 @@
 // item's model blob into shared memory with one bulk-async copy, and run its
 // trajectories thread-per-trajectory or warp-per-trajectory as the item
 // says (PYST_GROUPS: for batches too small to fill the GPU thread by thread,
-// a group of lanes per trajectory where the item's model allows it).  Replaces the reference's one-JIT-and-launch-sequence-per-model
-// sweep (examples/*_sim.py loops over CuTauLeaping().run, e.g.
-// examples/schlogl_sim.py:66-80).  Built once per PYST_SCORE flavour.
+// a group of lanes per trajectory where the item's model allows it).
+// Replaces the reference's one-JIT-and-launch-sequence-per-model sweep
+// (examples/*_sim.py loops over CuTauLeaping().run, e.g.
+// examples/schlogl_sim.py:66-80).  Built once per (PYST_GROUPS, PYST_SCORE)
+// flavour.
 #include "pyst_group.cuh"
 #include "pyst_launch.cuh"
 
@@ -119,7 +121,7 @@ __global__ void PYST_BATCH_BOUNDS
             const pyst_batch_item* __restrict__ items, int64_t n_items,
             RunArgs ra, OutBase ob, unsigned long long* queue, unsigned* done,
             int max_blob_words, int warp_bytes, int dyn_bytes, int pk_bytes,
-            int fd_bytes, int parts, int part, int wide_cap) {
+            int fd_bytes, int wide_cap) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ long long s_item;
   __shared__ int s_last;
@@ -146,21 +148,12 @@ __global__ void PYST_BATCH_BOUNDS
     if (threadIdx.x == 0) s_item = (long long)atomicAdd(queue, 1ull);
     __syncthreads();
     const long long it = s_item;
-    if (it >= n_items * parts) break;
-    pyst_batch_item item = items[PYST_GROUPS ? it / parts : it];
+    if (it >= n_items) break;
+    const pyst_batch_item item = items[it];
     // the model's trajectory count (a split model's chunks share it) and
     // this item's first trajectory in it
     const int64_t U = item.model_n_traj > 0 ? item.model_n_traj : item.n_traj;
-    int64_t cb = item.model_n_traj > 0 ? item.chunk_begin : 0;
-    int chunks = item.group_chunks > 1 ? item.group_chunks : 1;
-    if (PYST_GROUPS && parts > 1) {
-      // this block's part of the item: a chunk of the chunk
-      const int64_t lo = (it % parts) * (int64_t)part;
-      const int64_t left = item.n_traj - lo;
-      cb += lo;
-      item.n_traj = left < 0 ? 0 : left < part ? left : part;
-      chunks *= parts;
-    }
+    const int64_t cb = item.model_n_traj > 0 ? item.chunk_begin : 0;
     const uint32_t* blob = gblobs + item.blob_offset;
     const int words = (int)__ldg(blob + PYST_H_WORDS);
     const bool ok = stage_blob(sblob, blob, words, bar, parity,
@@ -195,11 +188,13 @@ __global__ void PYST_BATCH_BOUNDS
           packed_bytes(m.R) <= (size_t)pk_bytes) {
         // (uniform over the block: every thread reads the same item)
         m.pk = spk;
+#if !PYST_GROUPS
         if (fd_bytes && m.nlaw == 0 &&
             has_direct_forms(m.R, blob_direct_factors(sblob))) {
           m.fd = sfd;
           build_direct(m, sfd, bs);
         }
+#endif
         m.fast = __syncthreads_and(pack_reactions(m, spk)) != 0;
       }
       // (uniform: items beyond the register arrays, or warp-mapped)
@@ -209,13 +204,10 @@ __global__ void PYST_BATCH_BOUNDS
         if (__syncthreads_and(build_wide(m, sfw))) m.fw = sfw;
       const bool tau = item.method == PYST_METHOD_TAU_LEAP;
 #if PYST_GROUPS
-      // (block-uniform) 4 lanes per trajectory where reactions and species
-      // allow, else 8
-      const int factors =
+      // (block-uniform)
+      const int lanes =
           item.mapping == PYST_MAP_THREAD && m.nlaw == 0 && m.fast
-              ? blob_direct_factors(sblob) : 0;
-      const int lanes = factors < 1 || factors > 3 || m.S > 8 ? 0
-                        : m.R <= 4 && m.S <= 4 ? 4 : 8;
+              ? batch_lanes(blob_direct_factors(sblob), m.S, m.R) : 0;
       if (lanes) {
         auto out = [&](int64_t u) {
           return ob.at(item.sample_offset, u, item.traj_offset,
@@ -259,31 +251,40 @@ __global__ void PYST_BATCH_BOUNDS
           const TrajOut o = ob.at(item.sample_offset, u, item.traj_offset,
                                   item.score_offset, U, m.R);
           const uint64_t id = (uint64_t)item.traj_id_base + (uint64_t)u;
-          if (!PYST_GROUPS && direct) {
-            // (block-uniform) an item with direct forms: the reaction count
-            // (2 to 8) fixed at compile time, three factor slots (one form
-            // for all items keeps the kernel's size)
-#if !PYST_GROUPS
-            switch (m.R) {
-#define PYST_EXACT_CASE(r)                                                 \
+#define PYST_EXACT_CASE(r, fc)                                             \
   case r:                                                                  \
     if (tau)                                                               \
-      run_thread<r, true, SCORE, kPkPacked, r, 3>(m, xcol, slot, bs, ra,   \
-                                                  id, o);                  \
-    else                                                                   \
-      run_thread<r, false, SCORE, kPkPacked, r, 3>(m, xcol, slot, bs, ra,  \
+      run_thread<r, true, SCORE, kPkPacked, r, fc>(m, xcol, slot, bs, ra,  \
                                                    id, o);                 \
+    else                                                                   \
+      run_thread<r, false, SCORE, kPkPacked, r, fc>(m, xcol, slot, bs, ra, \
+                                                    id, o);                \
     break;
-              PYST_EXACT_CASE(2)
-              PYST_EXACT_CASE(3)
-              PYST_EXACT_CASE(4)
-              PYST_EXACT_CASE(5)
-              PYST_EXACT_CASE(6)
-              PYST_EXACT_CASE(7)
-              PYST_EXACT_CASE(8)
-#undef PYST_EXACT_CASE
-            }
+#define PYST_EXACT_CASES(fc)                                               \
+  switch (m.R) {                                                           \
+    PYST_EXACT_CASE(2, fc)                                                 \
+    PYST_EXACT_CASE(3, fc)                                                 \
+    PYST_EXACT_CASE(4, fc)                                                 \
+    PYST_EXACT_CASE(5, fc)                                                 \
+    PYST_EXACT_CASE(6, fc)                                                 \
+    PYST_EXACT_CASE(7, fc)                                                 \
+    PYST_EXACT_CASE(8, fc)                                                 \
+  }
+          // (block-uniform) a packable item of 2 to 8 reactions: the
+          // reaction count fixed at compile time, with three factor slots
+          // where it has direct forms (one form for all items keeps the
+          // kernel's size), else with packed descriptors (600 models x 128
+          // trajectories of 8 reactions, one of four factors, with scores:
+          // direct method 6.7 ms, tau-leaping 16.5; with a run-time count
+          // 7.8 and 18.0)
+          if (direct) {
+#if !PYST_GROUPS
+            PYST_EXACT_CASES(3)
 #endif
+          } else if (m.fast && m.R >= 2 && m.R <= 8) {
+            PYST_EXACT_CASES(0)
+#undef PYST_EXACT_CASES
+#undef PYST_EXACT_CASE
           } else if (m.R <= 8) {
             if (tau) run_thread<8, true, SCORE>(m, xcol, slot, bs, ra, id, o);
             else run_thread<8, false, SCORE>(m, xcol, slot, bs, ra, id, o);
@@ -313,14 +314,14 @@ __global__ void PYST_BATCH_BOUNDS
     if (ob.stats || ob.jac) {
       // a split model: every thread makes its outputs visible device-wide
       // before the chunk is counted (uniform branch)
-      if (chunks > 1) __threadfence();
+      if (item.group_chunks > 1) __threadfence();
       __syncthreads();  // the item's samples are all written
       bool last = true;
-      if (chunks > 1) {
+      if (item.group_chunks > 1) {
         // the block finishing the model's last chunk reduces the model
         if (threadIdx.x == 0) {
           s_last = atomicAdd(done + item.group, 1u) + 1u ==
-                   (unsigned)chunks;
+                   (unsigned)item.group_chunks;
           if (s_last) __threadfence();
         }
         __syncthreads();
@@ -352,7 +353,8 @@ int PYST_CAT(launch_batch_, PYST_GROUPS, PYST_SCORE)(
   if (smem > kMaxDynSmem) return PYST_EUNSUPPORTED;
   // room for the direct forms and their columns' extra element, if it fits
   const size_t fd = direct_bytes(kDirectMaxR), one = (size_t)bs * 4;
-  const size_t fd_bytes = smem + fd + one <= kMaxDynSmem ? fd : 0;
+  const size_t fd_bytes =
+      !PYST_GROUPS && smem + fd + one <= kMaxDynSmem ? fd : 0;
   if (fd_bytes) smem += fd + one;
   const size_t wide = (size_t)lim->max_reactions * 16;
   const int wide_cap = smem + wide <= kMaxDynSmem ? lim->max_reactions : 0;
@@ -366,19 +368,12 @@ int PYST_CAT(launch_batch_, PYST_GROUPS, PYST_SCORE)(
   int per_sm = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kf, bs, smem);
   if (per_sm < 1) per_sm = 1;
-  int parts = 1, part = 0;
-#if PYST_GROUPS
-  if (lim->reserved >> 16 > 1 && (lim->reserved & 0xFFFF) > 0) {
-    parts = lim->reserved >> 16;
-    part = lim->reserved & 0xFFFF;
-  }
-#endif
   int64_t grid = (int64_t)num_sms() * per_sm;
-  if (grid > n_items * parts) grid = n_items * parts;
+  if (grid > n_items) grid = n_items;
   kf<<<(unsigned)grid, bs, smem, st>>>(d_blobs, d_items, n_items, ra, ob,
                                        queue, done, lim->max_blob_words,
                                        (int)wb, (int)dyn, (int)pk_bytes,
-                                       (int)fd_bytes, parts, part, wide_cap);
+                                       (int)fd_bytes, wide_cap);
   return cudaGetLastError() == cudaSuccess ? PYST_OK : PYST_ECUDA;
 }
 
