@@ -9,7 +9,8 @@ each bucket present in a batch the tuner builds a small trial batch from up
 to ``sample`` of its models, times it with each mapping under a short step
 budget (events per second on the device, CUDA events), and keeps the
 faster.  The block size (64 or 128 threads) is chosen the same way on a
-sample of the whole batch.  Results are cached per GPU name in a JSON file
+sample of the whole batch.  Results are cached per GPU name and version of
+the kernels in a JSON file
 (``$PYST_AUTOTUNE_CACHE`` or ``~/.cache/py_stoch_b200/autotune.json``), so a
 bucket is measured once.
 
@@ -37,6 +38,13 @@ ROUNDS = ((16, 2), (20, 2), (32, 3), (40, 4), (50, 5), (64, 4), (100, 8))
 POOLS = (1, 2)
 SORTED_BLOCKS = (896, 448)
 
+DEFAULT_GEOMETRY = {'round_ssa': 0, 'round_leap': 0, 'pool_slots': 0,
+                    'sorted_block': 0}
+
+# Cache entries belong to the kernels they were measured with: raised when a
+# kernel's speed changes, so that older entries are measured again.
+KERNELS = 2
+
 _lock = threading.Lock()
 
 
@@ -62,7 +70,8 @@ class Autotuner(object):
                  budget=2000, score=False):
         torch = _torch()
         self.device = torch.device(device or 'cuda')
-        self.gpu = torch.cuda.get_device_name(self.device)
+        self.gpu = '%s, kernels %d' % (
+            torch.cuda.get_device_name(self.device), KERNELS)
         self.path = path or cache_path()
         self.sample = sample
         self.n_traj = n_traj
@@ -185,38 +194,49 @@ class Autotuner(object):
                 best = max(best, ev / max(st.elapsed_time(en), 1e-3) * 1e3)
         return best
 
+    @staticmethod
+    def _geometry_key(model, n_traj, method):
+        """Bucket of a single-model run: the model's, the run size's and
+        whether the library's own choice is the lane groups (the line lies
+        within a size bucket)."""
+        from .simulator import run_kernel
+        groups = run_kernel(model, n_traj, method=method)[0] == \
+            _lib.KERNEL_GROUP
+        return 'geom/%s/N%d%s' % (bucket(model, method),
+                                  _edge(int(n_traj), N_EDGES),
+                                  '/groups' if groups else '')
+
     def tune_geometry(self, model, n_traj, method='tau', force=False):
-        """Measure every candidate geometry of the mode-sorted scheduler on
-        ``n_traj`` trajectories of ``model`` (whole runs, events per second
-        by CUDA events, best of two after a warm-up) and cache the fastest
-        for the model's bucket and run size.  Returns the geometry dict
-        (keyword ``geometry`` of :func:`py_stoch_b200.simulator.simulate`).
+        """Measure the library's own choice (the lane groups for small runs of
+        small models, else the mode-sorted scheduler's default) and every
+        candidate geometry of the mode-sorted scheduler on ``n_traj``
+        trajectories of ``model`` (whole runs, events per second by CUDA
+        events, best of two after a warm-up) and cache the fastest for the
+        model's bucket and run size.  Returns the geometry dict (keyword
+        ``geometry`` of :func:`py_stoch_b200.simulator.simulate`), all zeros
+        for the library's own choice.
         """
-        key = 'geom/%s/N%d' % (bucket(model, method),
-                               _edge(int(n_traj), N_EDGES))
+        key = self._geometry_key(model, n_traj, method)
         if key in self.table and not force:
             return dict(self.table[key]['geometry'])
-        res = {}
+        cands = {'default': dict(DEFAULT_GEOMETRY)}
         for (rs, rl) in ROUNDS:
             for pool in POOLS:
                 for blk in SORTED_BLOCKS:
-                    g = {'round_ssa': rs, 'round_leap': rl,
-                         'pool_slots': pool, 'sorted_block': blk}
-                    name = '%d/%d/p%d/b%d' % (rs, rl, pool, blk)
-                    res[name] = (g, self._time_single(model, n_traj, method,
-                                                      g))
-        best = max(res, key=lambda k: res[k][1])
-        self.table[key] = {'geometry': res[best][0],
-                           'events_per_s': {k: v[1] for k, v in
-                                            res.items()}}
-        self.timings[key] = self.table[key]['events_per_s']
+                    cands['%d/%d/p%d/b%d' % (rs, rl, pool, blk)] = {
+                        'round_ssa': rs, 'round_leap': rl,
+                        'pool_slots': pool, 'sorted_block': blk}
+        res = {name: self._time_single(model, n_traj, method, g)
+               for name, g in cands.items()}
+        best = max(res, key=res.get)
+        self.table[key] = {'geometry': cands[best], 'events_per_s': res}
+        self.timings[key] = res
         self._save()
-        return dict(res[best][0])
+        return dict(cands[best])
 
     def geometry(self, model, n_traj, method='tau'):
         """Cached geometry for this model bucket and run size, or None."""
-        ent = self.table.get('geom/%s/N%d' % (bucket(model, method),
-                                              _edge(int(n_traj), N_EDGES)))
+        ent = self.table.get(self._geometry_key(model, n_traj, method))
         return dict(ent['geometry']) if ent else None
 
     # ---- lookup ----------------------------------------------------------

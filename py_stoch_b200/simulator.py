@@ -75,6 +75,24 @@ def device_blob(model, device):
     return torch.from_numpy(model.blob().view(np.int32)).to(device)
 
 
+def run_kernel(model, n_traj, method='direct', mapping='auto', score=False,
+               sorted_blocks=True, geometry=None):
+    """The kernel :func:`simulate` takes for a run (``_lib.KERNEL_*``) and its
+    lanes per trajectory.  Nothing is launched."""
+    geo = geometry or {}
+    r = _lib.RunDesc(int(n_traj), 0, 0, _method(method), _mapping(mapping),
+                     100, 63, 0, 0,
+                     0 if sorted_blocks else _lib.FLAG_UNSORTED,
+                     *(int(geo.get(k, 0)) for k in (
+                         'round_ssa', 'round_leap', 'pool_slots',
+                         'sorted_block')))
+    kernel, lanes = C.c_int32(0), C.c_int32(0)
+    _lib.check(_lib.lib().pyst_run_kernel(
+        model.blob().ctypes.data, C.byref(r), 1 if score else 0,
+        C.byref(kernel), C.byref(lanes)), 'pyst_run_kernel')
+    return kernel.value, lanes.value
+
+
 def simulate(model, n_traj, method='direct', seed=0, traj_id_base=0,
              mapping='auto', device=None, stream=None, status=True,
              events=True, seqhash=False, t_final=False, score=False,
