@@ -24,7 +24,9 @@ int pyst_test_philox(uint64_t seed, uint64_t id, uint64_t n0, int64_t count,
 int pyst_test_philox_raw(const uint32_t* d_ctr_key, int64_t count,
                          uint32_t* d_out, int use_curand, void* stream);
 
-/* which: 0 pyst_log, 1 pyst_exp, 2 log-factorial, 3 CUDA log, 4 CUDA exp. */
+/* which: 0 pyst_log, 1 pyst_exp, 2 log-factorial, 3 CUDA log, 4 CUDA exp.
+ * Of pairs (d_x holds 2 n doubles): the straight-line FP64 division (5) and
+ * CUDA's (6), the FP32 ones (7, 8), the uniform of two random words (9). */
 int pyst_test_math(const double* d_x, int64_t n, int which, double* d_out,
                    void* stream);
 

@@ -281,6 +281,14 @@ __global__ void k_math(const double* x, int64_t n, int which, double* out) {
   else if (which == 2) v = pyst_logfact(x[i]);
   else if (which == 3) v = log(x[i]);
   else if (which == 4) v = exp(x[i]);
+  // pairs: (a, b), or the two words of a uniform
+  else if (which == 5) v = ddiv_normal(x[2 * i], x[2 * i + 1]);
+  else if (which == 6) v = __ddiv_rn(x[2 * i], x[2 * i + 1]);
+  else if (which == 7)
+    v = (double)fdiv_normal((float)x[2 * i], (float)x[2 * i + 1]);
+  else if (which == 8)
+    v = (double)__fdiv_rn((float)x[2 * i], (float)x[2 * i + 1]);
+  else if (which == 9) v = u53((uint32_t)x[2 * i], (uint32_t)x[2 * i + 1]);
   out[i] = v;
 }
 
@@ -493,7 +501,7 @@ int pyst_test_philox_raw(const uint32_t* d_ctr_key, int64_t count,
 int pyst_test_math(const double* d_x, int64_t n, int which, double* d_out,
                    void* stream) {
   if (n <= 0) return PYST_OK;
-  if (!d_x || !d_out || which < 0 || which > 4) return PYST_EINVAL;
+  if (!d_x || !d_out || which < 0 || which > 9) return PYST_EINVAL;
   k_math<<<(unsigned)((n + 127) / 128), 128, 0, (cudaStream_t)stream>>>(
       d_x, n, which, d_out);
   return cudaGetLastError() == cudaSuccess ? PYST_OK : PYST_ECUDA;
