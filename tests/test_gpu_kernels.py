@@ -10,6 +10,7 @@ oracle, with and without scores.
 import numpy as np
 import pytest
 
+from py_stoch_b200 import _lib, networks
 from py_stoch_b200.model import Model
 
 pytestmark = pytest.mark.gpu
@@ -64,8 +65,16 @@ def compare(g, o, n):
                                        err_msg=key)
 
 
-def check(torch, m, o, n, method, seed, **kw):
+def kernel(m, n, method, score=False, **kw):
+    from py_stoch_b200.simulator import run_kernel
+    return run_kernel(m, n, method, 'thread', score, **kw)[0]
+
+
+def check(torch, m, o, n, method, seed, want=None, **kw):
     from py_stoch_b200.simulator import simulate
+    route = {k: v for k, v in kw.items()
+             if k in ('score', 'geometry', 'sorted_blocks')}
+    assert want is None or kernel(m, n, method, **route) == want
     r = simulate(m, n, method=method, seed=seed, seqhash=True, t_final=True,
                  mapping='thread', **kw)
     torch.cuda.synchronize()
@@ -99,16 +108,19 @@ def test_small_packable(torch_cuda, built_lib, oracle_mod, factors, R, S,
     # 32, 32, 16, 8 and 4 or 8 lanes, a thread per trajectory (148 SMs; with
     # 9 or more species 16 or 32 lanes, then a thread)
     for n in (1, 300, 1700, 3001, 9000, MANY):
+        want = (_lib.KERNEL_GROUP if n <= 300 else None if n < MANY else
+                _lib.KERNEL_THREAD if method == 'direct' else
+                _lib.KERNEL_SORTED)
         for score in (False, True):
-            check(torch_cuda, m, o, n, method, seed, score=score)
+            check(torch_cuda, m, o, n, method, seed, want, score=score)
     if method == 'tau':
         for score in (False, True):
-            check(torch_cuda, m, o, 2500, method, seed, score=score,
-                  geometry={'round_ssa': 20, 'round_leap': 2})
-            check(torch_cuda, m, o, 2500, method, seed, score=score,
-                  geometry={'sorted_block': 448})
-            check(torch_cuda, m, o, 2500, method, seed, score=score,
-                  sorted_blocks=False)
+            for geo in ({'round_ssa': 20, 'round_leap': 2},
+                        {'sorted_block': 448}):
+                check(torch_cuda, m, o, 2500, method, seed,
+                      _lib.KERNEL_SORTED, score=score, geometry=geo)
+            check(torch_cuda, m, o, 2500, method, seed, _lib.KERNEL_THREAD,
+                  score=score, sorted_blocks=False)
     for chunk in (0, 128):  # a thread per trajectory, lane groups
         for score in (False, True):
             b = Batch([m], 300, method=method, mapping='thread', score=score,
@@ -131,3 +143,75 @@ def test_register_engine(torch_cuda, built_lib, oracle_mod, R, lists, method):
         for kw in ({},) if method == 'direct' else (
                 {'sorted_blocks': False}, {'geometry': {'round_ssa': 30}}):
             check(torch_cuda, m, o, n, method, R, score=score, **kw)
+
+
+def test_ends_under_every_scheduler(torch_cuda, built_lib, oracle_mod):
+    """Many sample times per step, counts that leave the int32 range,
+    absorption and the step budget, in the thread kernels, the simple tau loop
+    and the mode-sorted scheduler (direct forms, packed and lists)."""
+    t = np.linspace(0, 20, 9).astype(np.float32)
+    decay = [[1, 0], [0, 1]], [[0, 0], [1, 0]]
+    grow = [[1, 0], [0, 1]], [[2, 0], [0, 2]]
+    models = [
+        (networks.schlogl(t_end=0.05, n_samples=300), {}),
+        (networks.schlogl(t_end=0.05, n_samples=50), {'step_budget': 33}),
+        (Model.mass_action(*decay, [3.0, 2.0], [30, 20], t), {}),
+        (Model.mass_action(*decay, [3.0, 2.0], [30, 20], t),
+         {'step_budget': 7}),
+        (Model.mass_action(*grow, [40.0, 1.0], [2**31 - 40, 7],
+                           np.float32([0, 1e-10, 3e-10])), {}),
+        # four factors: packed descriptors
+        (Model.mass_action([[1, 2], [0, 2]], [[2, 1], [0, 3]], [40.0, 1e-12],
+                           [2**31 - 40, 9],
+                           np.float32([0, 1e-10, 3e-10])), {}),
+        # a change of 20: lists
+        (Model.mass_action([[1, 0], [0, 1]], [[21, 0], [0, 0]], [40.0, 1.0],
+                           [2**31 - 400, 9],
+                           np.float32([0, 1e-10, 3e-10])), {})]
+    assert [packable(built_lib, m) for m, _ in models] == [1] * 6 + [0]
+    for m, kw in models:
+        o = oracle_mod.simulate(m, MANY, 0, seed=8, **kw)
+        for score in (False, True):
+            check(torch_cuda, m, o, MANY, 'direct', 8, _lib.KERNEL_THREAD,
+                  score=score, **kw)
+        o = oracle_mod.simulate(m, MANY, 1, seed=8, **kw)
+        for score in (False, True):
+            for n, geo in ((MANY, {}), (700, {'round_ssa': 3}),
+                           (700, {'pool_slots': 1})):
+                check(torch_cuda, m, o, n, 'tau', 8, _lib.KERNEL_SORTED,
+                      score=score, geometry=geo, **kw)
+            check(torch_cuda, m, o, 700, 'tau', 8, _lib.KERNEL_THREAD,
+                  score=score, sorted_blocks=False, **kw)
+
+
+def test_staging_timeout_of_the_kernel_named(torch_cuda, built_lib):
+    """Every kernel marks its trajectories when the model's staging gives up
+    (the copy itself still lands)."""
+    from py_stoch_b200.batch import Batch
+    from py_stoch_b200.simulator import simulate
+    m = model(2, 3)
+    other = model(2, 3, lists=True)
+    runs = [(m, 64, 'direct', _lib.KERNEL_GROUP, {}),
+            (m, 3000, 'tau', _lib.KERNEL_GROUP, {}),
+            (m, MANY, 'direct', _lib.KERNEL_THREAD, {}),
+            (m, MANY, 'tau', _lib.KERNEL_SORTED, {}),
+            (m, 3000, 'tau', _lib.KERNEL_SORTED,
+             {'geometry': {'round_ssa': 40}}),
+            (m, 3000, 'tau', _lib.KERNEL_THREAD, {'sorted_blocks': False}),
+            (other, 300, 'direct', _lib.KERNEL_LOCKSTEP, {}),
+            (other, 3000, 'tau', _lib.KERNEL_SORTED, {})]
+    built_lib.pyst_test_set_staging_polls(0)
+    try:
+        for mm, n, method, want, kw in runs:
+            assert kernel(mm, n, method, **kw) == want
+            r = simulate(mm, n, method=method, mapping='thread', **kw)
+            torch_cuda.cuda.synchronize()
+            assert (r['status'].cpu().numpy() == _lib.TRAJ_STAGING).all()
+        for chunk in (0, 128):
+            b = Batch([m, other], 200, method='tau', chunk=chunk)
+            assert b.lane_groups == (chunk > 0)
+            b.run(seed=1)
+            torch_cuda.cuda.synchronize()
+            assert (b.out['status'].cpu().numpy() == _lib.TRAJ_STAGING).all()
+    finally:
+        built_lib.pyst_test_set_staging_polls(-1)
