@@ -125,23 +125,33 @@ OutBase make_outbase(const pyst_outputs* out, int64_t n_traj) {
 // Lanes per trajectory for a run of n trajectories (pyst_group.cuh), or 0 for
 // a thread per trajectory.  More lanes shorten a step while warps are few;
 // past that they cost issue slots.  The lines, in trajectories per SM, lie
-// where the next form measured faster (148 SMs, ms, four steps per vote; t:
-// thread form, for tau-leaping the mode-sorted scheduler):
-//   direct, Lotka-Volterra: 1,184 32: 53 16: 48; 2,368 16: 55 8: 52;
-//     4,999 8: 70 4: 68 t: 119; 9,472 4: 70 t: 121; 20,011 4: 147 t: 142;
-//   direct, telegraph (6 reactions): 592 32: 2.0 16: 2.2; 2,368 16: 2.4
-//     8: 2.4; 9,472 8: 3.7 t: 5.0; 20,011 8: 7.1 t: 5.8;
-//   tau, Schlogl: 2,368 32: 5.1 16: 6.9; 4,999 32: 10.8 8: 9.4 4: 9.5;
-//     20,011 4: 15.6 t: 20.3; 40,000 4: 31.9 t: 20.3;
-//   tau, Lotka-Volterra: 2,368 32: 21.0 8: 20.9; 9,472 8: 27 4: 25;
-//     20,011 4: 33 t: 90; 40,000 4: 54 t: 93.
+// near where the next form is the faster one, on most of seven models (148
+// SMs, ms; lanes or t, a thread each, for tau-leaping the mode-sorted
+// scheduler):
+//   direct, Schlogl: 8 32: 2.4 16: 2.6; 16 16: 2.7 8: 3.0; 32 8: 3.4 4: 4.0;
+//     64 8: 4.6 4: 4.5; 112 4: 5.5 t: 7.5; 240 4: 7.9 t: 8.8;
+//   direct, Lotka-Volterra: 8 32: 4.3 16: 4.2; 16 16: 4.9 8: 4.7; 32 8: 5.5
+//     4: 6.4; 64 8: 8.3 4: 7.3; 112 4: 10.9 t: 12.9; 144 4: 15.9 t: 15.1;
+//   direct, telegraph (6 reactions): 8 32: 0.37 16: 0.40; 24 16: 0.49 8: 0.56;
+//     80 8: 0.89 t: 0.98; 96 8: 1.05 t: 1.01;
+//   direct, 8 reactions and species: 16 16: 0.32 8: 0.26; 64 8: 0.43 t: 0.55;
+//     80 8: 0.63 t: 0.55;
+//   tau, Schlogl: 16 32: 2.0 8: 2.5; 32 8: 3.1 4: 3.3; 160 4: 7.4 t: 7.9; 192
+//     4: 8.6 t: 7.7;
+//   tau, Lotka-Volterra: 16 32: 0.54 8: 0.52; 32 8: 0.55 4: 0.56; 160 4: 1.0
+//     t: 1.8; 240 4: 1.1 t: 1.8;
+//   tau, telegraph: 16 32: 0.57 16: 0.53; 96 8: 1.3 t: 1.9; 160 8: 1.9 t: 2.0;
+//   tau, 8 reactions and species: 16 32: 0.36 8: 0.28; 96 8: 0.74 t: 0.75;
+//   14 species: direct 32 16: 0.35 t: 0.52; 48 16: 0.55 t: 0.52; tau 32 16:
+//     0.36 t: 0.81; 64 16: 0.77 t: 0.81; 20 species: direct 16 32: 0.23 t:
+//     0.54; 32 32: 0.42 t: 0.41; tau 16 32: 0.24 t: 0.71; 64 32: 0.84 t: 0.72.
 int group_lanes(const HostModelInfo& mi, int64_t n, bool tau) {
   if (mi.factors < 1 || mi.S > 32) return 0;
   int least = mi.R > 4 || mi.S > 4 ? 8 : 4;
   while (least < mi.S) least *= 2;
   const int64_t per_sm = (n + num_sms() - 1) / num_sms();
   if (per_sm <= (tau ? 16 : 8)) return 32;
-  if (least <= 16 && per_sm <= (tau ? 16 : 12)) return 16;
+  if (!tau && least <= 16 && per_sm <= 12) return 16;
   if (least <= 8 && per_sm <= 32) return 8;
   const int most = least == 4 ? (tau ? 160 : 112)
                    : least == 8 ? (tau ? 96 : 80)

@@ -3,7 +3,7 @@
 //
 // A trajectory is one dependent chain of steps, so a run of few trajectories
 // is bound by the latency of a step (about 4 cycles per instruction of a
-// lone warp), not by issue.  Here LG adjacent lanes (8 or 32) share a
+// lone warp), not by issue.  Here LG adjacent lanes (4 to 32) share a
 // trajectory, and a step's chain is what remains when its work is laid out
 // over them, with no shared memory on it:
 //   * lane j owns reaction j: it holds the rate, the counts of the (up to
@@ -28,10 +28,10 @@
 // Measured (one B200, ms; before: the mode-sorted scheduler for tau-leaping,
 // a warp-wide tree of speculated steps for the direct method up to 2,368
 // trajectories, a thread each above): tau Schlogl 4,999 trajectories 20.2 ->
-// 9.0, 1,184 20.3 -> 3.9; tau Lotka-Volterra 20,011 85 -> 32, 1,184 75 -> 17;
-// direct Lotka-Volterra 1,024 72 -> 40, 4,700 119 -> 47; direct telegraph
+// 9.3, 1,184 20.3 -> 3.9; tau Lotka-Volterra 20,011 85 -> 31, 1,184 75 -> 17;
+// direct Lotka-Volterra 1,024 72 -> 41, 4,700 119 -> 47; direct telegraph
 // 1,024 7.6 -> 1.6; a 64-set sweep of 256 trajectories with scores 236 ->
-// 125.  A step takes about 210 cycles of a lone warp, a leap about 4,000; past
+// 123.  A step takes about 210 cycles of a lone warp, a leap about 4,000; past
 // 4 lanes x 112 trajectories per SM issue bounds it.
 //
 // Same algorithms and reference sources as pyst_engine.cuh.  Models: at most

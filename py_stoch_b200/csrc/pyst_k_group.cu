@@ -75,6 +75,9 @@ int launch_one(const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
   return cudaGetLastError() == cudaSuccess ? PYST_OK : PYST_ECUDA;
 }
 
+// (16 lanes in tau-leaping: models of 9 to 16 species only.  Six factor slots:
+// models of four to six factors, 32 trajectories per SM, 6 reactions: 0.44 ms
+// against 1.22 for a thread each, tau-leaping 0.63 against 2.12.)
 template <int R, int FC>
 int launch_lanes(int lanes, const uint32_t* d_blob, const HostModelInfo& mi,
                  int64_t n, uint64_t id_base, const RunArgs& ra,

@@ -16,7 +16,7 @@
 // once, so no long trajectory starts late, and the mode mix of a round can
 // be chosen from a larger set.  Per-trajectory arithmetic is exactly that of
 // run_thread, so results do not depend on the schedule.  Built once per
-// PYST_SCORE flavour.
+// (PYST_SCORE, PYST_PART).
 #include "pyst_launch.cuh"
 
 namespace pyst {
@@ -67,10 +67,10 @@ constexpr int kPrefBlock =
 // (128 / 8 100, 256 / 16 107, 256 / 32 121, earlier kernels), and resizing
 // leap rounds to match the SSA rounds' measured time was slower too.
 // With direct forms a leap costs about ten steps (FP32 sampler), and whole
-// fallback rounds of 100 with 8 leaps are the better default, ms against
-// 40 / 4: Schlogl 262,144 39.0, 39.9; 60,000 20.6, 21.3; Lotka-Volterra
-// 65,536 95.7, 99.0; telegraph 65,536 13.1, 14.9; small models that only leap
-// 4 reactions, 150,000 1.39, 1.28; 8 reactions 2.58, 2.45.  Other models'
+// fallback rounds of 100 with 8 leaps are the default, ms against 40 / 4:
+// Schlogl 262,144 39.0, 39.9; 60,000 20.6, 21.3; Lotka-Volterra 65,536 95.7,
+// 99.0; telegraph 65,536 13.1, 14.9; but models that only leap, 150,000, 4
+// reactions 1.39, 1.28; 8 reactions 2.58, 2.45.  Other models'
 // leaps are longer and gather in few rounds, 100 / 8 against 40 / 4: lists of
 // 4 reactions, 150,000 3.22, 2.66, of 8 7.1, 6.0; packable, 9 reactions 6.2,
 // 5.2; 16 reactions 11.1, 10.1; 400,000 30.8, 28.4.

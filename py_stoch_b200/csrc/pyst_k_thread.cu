@@ -203,7 +203,10 @@ int launch_one(const uint32_t* d_blob, const HostModelInfo& mi, int64_t n,
                                  kPkPacked>
                 : k_plain_thread<MR, (bool)PYST_TAU, (bool)PYST_SCORE,
                                  kPkLists>;
-  // a large network's reaction words, if they fit
+  // a large network's reaction words, if they fit (100 to 1,000 reactions,
+  // about the most a blob holds, 2,000 and 20,000 trajectories: direct method
+  // 3.1 to 4.1 times as fast, tau-leaping 1.04 to 1.08 times; none slower for
+  // the shared memory they take)
   const bool wide = MR == 0 && mi.nlaw == 0 &&
                     smem + (size_t)mi.R * 16 <= kMaxDynSmem;
   if (wide) smem += (size_t)mi.R * 16;

@@ -69,7 +69,8 @@ int PYST_CAT(launch_plain_warp_, PYST_TAU, PYST_SCORE)(
   const size_t wb = host_warp_bytes(mi.S, mi.R, PYST_SCORE);
   size_t smem = (size_t)mi.words * 4 + 16 + wb * nw;
   if (smem > kMaxDynSmem) return PYST_EUNSUPPORTED;
-  // the reaction words, if they fit
+  // the reaction words, if they fit (100 to 1,000 reactions, 500 and 5,000
+  // trajectories: 1.7 to 3.7 times as fast)
   const bool wide =
       mi.nlaw == 0 && smem + (size_t)mi.R * 16 <= kMaxDynSmem;
   if (wide) smem += (size_t)mi.R * 16;
