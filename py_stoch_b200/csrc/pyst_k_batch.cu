@@ -115,6 +115,33 @@ __device__ void item_epilogue(const ModelView& m, const pyst_batch_item& item,
   }
 }
 
+#if !PYST_GROUPS
+// One trajectory of an item with direct forms.  The tau-leaping forms are
+// functions of their own (arguments by value: the model view stays in
+// registers), except scored ones of more than 4 reactions: inlined into this
+// large kernel their spills depended on what else was in it (2,048 sweep sets
+// x 256 trajectories, ms, inlined and out of line: 809 and 617, with scores
+// 747 and 697; 600 telegraph and 600 Schlogl models of 256 with scores 35 and
+// 41 with the 6-reaction form out of line too; the direct method with scores
+// 14 and 22).
+template <int R, bool TAU, bool SCORE>
+__device__ __noinline__ void run_exact_call(ModelView m, int32_t* xcol,
+                                            int64_t* slot, int bs, RunArgs ra,
+                                            uint64_t id, TrajOut o) {
+  run_thread<R, TAU, SCORE, kPkPacked, R, 3>(m, xcol, slot, bs, ra, id, o);
+}
+template <int R, bool TAU, bool SCORE>
+__device__ __forceinline__ void run_exact(const ModelView& m, int32_t* xcol,
+                                          int64_t* slot, int bs,
+                                          const RunArgs& ra, uint64_t id,
+                                          const TrajOut& o) {
+  if constexpr (TAU && (!SCORE || R <= 4))
+    run_exact_call<R, TAU, SCORE>(m, xcol, slot, bs, ra, id, o);
+  else
+    run_thread<R, TAU, SCORE, kPkPacked, R, 3>(m, xcol, slot, bs, ra, id, o);
+}
+#endif
+
 template <bool SCORE>
 __global__ void PYST_BATCH_BOUNDS
     k_batch(const uint32_t* __restrict__ gblobs,
@@ -251,40 +278,29 @@ __global__ void PYST_BATCH_BOUNDS
           const TrajOut o = ob.at(item.sample_offset, u, item.traj_offset,
                                   item.score_offset, U, m.R);
           const uint64_t id = (uint64_t)item.traj_id_base + (uint64_t)u;
-#define PYST_EXACT_CASE(r, fc)                                             \
+          if (direct) {
+            // (block-uniform) an item with direct forms: the reaction count
+            // (2 to 8) fixed at compile time, three factor slots (one form
+            // for all items keeps the kernel's size)
+#if !PYST_GROUPS
+            switch (m.R) {
+#define PYST_EXACT_CASE(r)                                                 \
   case r:                                                                  \
     if (tau)                                                               \
-      run_thread<r, true, SCORE, kPkPacked, r, fc>(m, xcol, slot, bs, ra,  \
-                                                   id, o);                 \
+      run_exact<r, true, SCORE>(m, xcol, slot, bs, ra, id, o);             \
     else                                                                   \
-      run_thread<r, false, SCORE, kPkPacked, r, fc>(m, xcol, slot, bs, ra, \
-                                                    id, o);                \
+      run_exact<r, false, SCORE>(m, xcol, slot, bs, ra, id, o);            \
     break;
-#define PYST_EXACT_CASES(fc)                                               \
-  switch (m.R) {                                                           \
-    PYST_EXACT_CASE(2, fc)                                                 \
-    PYST_EXACT_CASE(3, fc)                                                 \
-    PYST_EXACT_CASE(4, fc)                                                 \
-    PYST_EXACT_CASE(5, fc)                                                 \
-    PYST_EXACT_CASE(6, fc)                                                 \
-    PYST_EXACT_CASE(7, fc)                                                 \
-    PYST_EXACT_CASE(8, fc)                                                 \
-  }
-          // (block-uniform) a packable item of 2 to 8 reactions: the
-          // reaction count fixed at compile time, with three factor slots
-          // where it has direct forms (one form for all items keeps the
-          // kernel's size), else with packed descriptors (600 models x 128
-          // trajectories of 8 reactions, one of four factors, with scores:
-          // direct method 6.7 ms, tau-leaping 16.5; with a run-time count
-          // 7.8 and 18.0)
-          if (direct) {
-#if !PYST_GROUPS
-            PYST_EXACT_CASES(3)
-#endif
-          } else if (m.fast && m.R >= 2 && m.R <= 8) {
-            PYST_EXACT_CASES(0)
-#undef PYST_EXACT_CASES
+              PYST_EXACT_CASE(2)
+              PYST_EXACT_CASE(3)
+              PYST_EXACT_CASE(4)
+              PYST_EXACT_CASE(5)
+              PYST_EXACT_CASE(6)
+              PYST_EXACT_CASE(7)
+              PYST_EXACT_CASE(8)
 #undef PYST_EXACT_CASE
+            }
+#endif
           } else if (m.R <= 8) {
             if (tau) run_thread<8, true, SCORE>(m, xcol, slot, bs, ra, id, o);
             else run_thread<8, false, SCORE>(m, xcol, slot, bs, ra, id, o);
