@@ -12,15 +12,18 @@
 #include "pyst_group.cuh"
 #include "pyst_launch.cuh"
 
-// Blocks of 128 threads per SM the register allocation must allow: 6 (at
-// most 80 registers) measured 11% faster than no bound on the
-// Schlogl/Lotka-Volterra sweep (2048 models, scores, statistics) and 1.5%
-// slower on synthetic networks of up to 256 reactions; 0 leaves it open.
+// Blocks of 128 threads per SM the register allocation must allow: 6 (at most
+// 80 registers) measured 11% faster than no bound on the Schlogl /
+// Lotka-Volterra sweep (2,048 models, scores, statistics) and 1.5% slower on
+// synthetic networks of up to 256 reactions, with every form inlined; with
+// the tau-leaping forms out of line scored batches take 5 (at most 96: 40
+// models of 10 to 24 reactions x 250 trajectories, tau-leaping 26.9 -> 19.4
+// ms, direct method 20.0 -> 18.2; the sweep 719 -> 712).
 #ifndef PYST_BATCH_MINB
 #if PYST_GROUPS
 #define PYST_BATCH_MINB 4  // as k_group
 #else
-#define PYST_BATCH_MINB 6
+#define PYST_BATCH_MINB (PYST_SCORE ? 5 : 6)
 #endif
 #endif
 #if PYST_BATCH_MINB > 0
@@ -118,12 +121,10 @@ __device__ void item_epilogue(const ModelView& m, const pyst_batch_item& item,
 #if !PYST_GROUPS
 // One trajectory of an item with direct forms.  The tau-leaping forms are
 // functions of their own (arguments by value: the model view stays in
-// registers), except scored ones of more than 4 reactions: inlined into this
-// large kernel their spills depended on what else was in it (2,048 sweep sets
-// x 256 trajectories, ms, inlined and out of line: 809 and 617, with scores
-// 747 and 697; 600 telegraph and 600 Schlogl models of 256 with scores 35 and
-// 41 with the 6-reaction form out of line too; the direct method with scores
-// 14 and 22).
+// registers): inlined into this large kernel their spills depended on what
+// else was in it (2,048 sweep sets x 256 trajectories, ms, inlined and out of
+// line: 809 and 615, with scores 747 and 712; the direct method with scores
+// loses, 600 telegraph and 600 Schlogl models of 256 14 and 22).
 template <int R, bool TAU, bool SCORE>
 __device__ __noinline__ void run_exact_call(ModelView m, int32_t* xcol,
                                             int64_t* slot, int bs, RunArgs ra,
@@ -135,7 +136,7 @@ __device__ __forceinline__ void run_exact(const ModelView& m, int32_t* xcol,
                                           int64_t* slot, int bs,
                                           const RunArgs& ra, uint64_t id,
                                           const TrajOut& o) {
-  if constexpr (TAU && (!SCORE || R <= 4))
+  if constexpr (TAU)
     run_exact_call<R, TAU, SCORE>(m, xcol, slot, bs, ra, id, o);
   else
     run_thread<R, TAU, SCORE, kPkPacked, R, 3>(m, xcol, slot, bs, ra, id, o);
