@@ -50,8 +50,8 @@ def workloads():
             # from one ncu capture of the simulation kernel on 229,376
             # trajectories: DRAM read + write per trajectory, and warp
             # instructions per reaction event
-            dram_bytes_per_traj=(540.65e6 + 1157.17e6) / 229376,
-            warp_inst_per_event=24014883287 / 4209068063),
+            dram_bytes_per_traj=(538.63e6 + 1146.28e6) / 229376,
+            warp_inst_per_event=23805063885 / 4209068063),
         'lv_ssa': dict(
             model=networks.lotka_volterra(), n=1024, method='direct',
             desc='plain Gillespie direct method, Lotka-Volterra (k1=10, '
